@@ -154,7 +154,7 @@ struct h3d_handle {
     float *f0 = nullptr;        // level-0 right-hand side of the refined mode [18][nv0]
     float *q = nullptr;         // level-1 Galerkin sub-element matrices
     double *d_ked = nullptr;
-    double *aug = nullptr;      // coarsest [K | K^-1]
+    double *aug = nullptr;      // coarsest K^-1 and the factorisation's scratch
     int ndof = 0;
     int *d_flag = nullptr;
     double *partial = nullptr;  // reduction scratch
@@ -168,7 +168,7 @@ struct h3d_handle {
     cudaGraphExec_t rgraph = nullptr;   // refinement step: u64 += u, f = f0 - K u64 (FP32 products)
     cudaGraphExec_t xgraph = nullptr;   // the same with the FP64-accumulated residual
     cudaGraphExec_t sgraph = nullptr;   // a solve's V-cycle: vgraph + rigid-translation deflation
-    cudaGraphExec_t fgraph = nullptr;   // coarsest assembly + Gauss-Jordan inverse (n + 1 launches)
+    cudaGraphExec_t fgraph = nullptr;   // coarsest assembly + Gauss-Jordan inverse (one launch per panel)
     cudaGraphExec_t dgraph = nullptr;   // design step (h3d_design_step)
     float *d_dcw = nullptr, *h_dcw = nullptr;  // sensitivity weights: device copy, pinned host source
     h3d_design_params dkey{};           // parameters and buffers the design graph was captured for

@@ -161,6 +161,60 @@ __device__ __forceinline__ const T &stage_args(const T &src, unsigned *buf) {
     return *reinterpret_cast<const T *>(buf);
 }
 #endif
+// ---- coarsest solve: x = K^-1 b ------------------------------------------------
+// Rows blk * (warps per CTA) + warp, then every nblk CTAs' worth, of u = K^-1 f for
+// the six load cases (project: the mean of each component removed from f first).
+// b: 6 n floats of shared memory.  A warp forms the six products of a row from one
+// read of it, each lane over the columns lane + 32 t, then a shuffle tree: the same
+// sums for any number of warps or CTAs.  CG: f through L2 (written earlier in the same
+// launch).  Every thread of the CTA must call it.
+constexpr int COARSEST_T = 256;
+inline size_t coarsest_smem(int n) { return sizeof(float) * NCASE * (size_t)n; }
+#ifdef __CUDACC__
+template <bool CG>
+__device__ __forceinline__ void coarsest_rows(const Planes &C, const double *__restrict__ inv, int n, int project,
+                                              const float *f, float *u, float *b, int blk, int nblk) {
+    __shared__ double mean[NF];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nv = n / 3;
+    const int n0 = C.n[0], n1 = C.n[1];
+    for (int v = threadIdx.x; v < nv; v += blockDim.x) {
+        const float *src = f + fidx(0, vidx(C, v % n0, v / n0 % n1, v / (n0 * n1)));
+#pragma unroll
+        for (int q = 0; q < NF; ++q)
+            b[(q / 3) * n + 3 * v + q % 3] = CG ? __ldcg(src + q * FVB) : __ldg(src + q * FVB);
+    }
+    if (threadIdx.x < NF) mean[threadIdx.x] = 0.0;
+    __syncthreads();
+    if (project) {
+        for (int q = wid; q < NF; q += nw) {
+            double s = 0;
+            for (int v = lane; v < nv; v += 32) s += (double)b[(q / 3) * n + 3 * v + q % 3];
+            s = warp_sum(s);
+            if (lane == 0) mean[q] = s / (double)nv;
+        }
+        __syncthreads();
+    }
+    for (int i = blk * nw + wid; i < n; i += nblk * nw) {
+        const double *row = inv + (long long)i * n;
+        double s[NCASE] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) {
+            const double k = __ldg(row + j);
+#pragma unroll
+            for (int c = 0; c < NCASE; ++c) s[c] = fma(k, (double)b[c * n + j] - mean[3 * c + j % 3], s[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < NCASE; ++c) s[c] = warp_sum(s[c]);
+        if (lane == 0) {
+            const int v = i / 3, m = i % 3;
+            float *o = u + fidx(m, vidx(C, v % n0, v / n0 % n1, v / (n0 * n1)));
+#pragma unroll
+            for (int c = 0; c < NCASE; ++c) o[3 * c * FVB] = (float)s[c];
+        }
+    }
+}
+#endif
+
 // host view of one device table: its address, slot count and launch sizes
 struct BatchTab {
     void *dev = nullptr;
@@ -291,8 +345,8 @@ void launch_dirichlet_patch(const Level &F, const Level &C, const float *rho, co
                             cudaStream_t s);
 void launch_galerkin(const Level &F, const Level &C, cudaStream_t s);
 void launch_coarse_assemble(const Level &C, double *aug, cudaStream_t s);
-// aug must hold gauss_jordan_doubles(n) doubles: the [n][2n] matrix and the
-// elimination scratch behind it
+// aug must hold gauss_jordan_doubles(n) doubles: two n x n buffers and the elimination
+// scratch behind them; the inverse ends in the first, row-major
 size_t gauss_jordan_doubles(int n);
 void launch_gauss_jordan(double *aug, int n, int *flag, cudaStream_t s);
 void launch_coarse_apply(const Level &C, const double *aug, int project, cudaStream_t s);
@@ -391,7 +445,7 @@ void launch_prolong_batch(const BatchTab &t, const int *active, int is_root, cud
 // (the same two-stage order as launch_norm_finish above NORM_FINISH_DIRECT blocks)
 int norm_batch_create(double *const *partial, const int *nblk, const int *design, int n, BatchTab *out);
 void launch_norm_finish_batch(const BatchTab &t, const int *active, double *out, cudaStream_t s);
-// the coarsest solve of each design (aug[i]: its [K | K^-1])
+// the coarsest solve of each design (aug[i]: its K^-1)
 int coarsest_batch_create(const Level *const *lv, const double *const *aug, const int *design, int n, BatchTab *out);
 void launch_coarse_apply_batch(const BatchTab &t, const int *active, int project, cudaStream_t s);
 // field conversion (k_coarse.cu)

@@ -700,7 +700,7 @@ struct BottomArgs {
     int nlv;                       // levels from `first` to the coarsest
     int project;                   // coarsest: remove the mean first
     int ndof;                      // coarsest unknowns
-    const double *aug;             // coarsest [K | K^-1]
+    const double *aug;             // coarsest K^-1
     unsigned *bar;                 // [0] arrivals, [1] generation
     int *flag;
 };
@@ -888,47 +888,15 @@ __device__ void bottom_residual(const CoarseArgs &a) {
     }
 }
 
-// the dense coarsest solve, one CTA per load case (the arithmetic of k_coarse_apply)
-__device__ void bottom_coarsest(const BottomArgs &A, double *b) {
+// the dense coarsest solve (the rows of k_coarse_apply, dealt to this grid's warps)
+__device__ void bottom_coarsest(const BottomArgs &A, float *b) {
     const CoarseArgs &a = A.lv[A.nlv];
-    const Planes &C = A.P[A.nlv];
-    const int n = A.ndof;
-    __shared__ double mean[3];
-    for (int c = blockIdx.x; c < NCASE; c += gridDim.x) {
-        for (int i = threadIdx.x; i < n; i += BOT_T) {
-            const long long lex = i / 3;
-            const int comp = i % 3;
-            const int x = (int)(lex % C.n[0]), y = (int)((lex / C.n[0]) % C.n[1]),
-                      z = (int)(lex / ((long long)C.n[0] * C.n[1]));
-            b[i] = __ldcg(a.f + fidx(3 * c + comp, vidx(C, x, y, z)));
-        }
-        __syncthreads();
-        if (threadIdx.x < 3) {
-            double sum = 0;
-            if (A.project)
-                for (int i = threadIdx.x; i < n; i += 3) sum += b[i];
-            mean[threadIdx.x] = sum / (double)(n / 3);
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += BOT_T) b[i] -= mean[i % 3];
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += BOT_T) {
-            const double *row = A.aug + (long long)i * 2 * n + n;
-            double sum = 0;
-            for (int j = 0; j < n; j++) sum = fma(row[j], b[j], sum);
-            const long long lex = i / 3;
-            const int comp = i % 3;
-            const int x = (int)(lex % C.n[0]), y = (int)((lex / C.n[0]) % C.n[1]),
-                      z = (int)(lex / ((long long)C.n[0] * C.n[1]));
-            a.u[fidx(3 * c + comp, vidx(C, x, y, z))] = (float)sum;
-        }
-        __syncthreads();
-    }
+    coarsest_rows<true>(A.P[A.nlv], A.aug, A.ndof, A.project, a.f, a.u, b, blockIdx.x, gridDim.x);
 }
 
 template <bool F32>
 __global__ void __launch_bounds__(BOT_T) k_vcycle_bottom(const __grid_constant__ BottomArgs A) {
-    extern __shared__ double bot_b[];
+    extern __shared__ float bot_b[];
     const int L = A.nlv;  // lv[1..L-1] smoothed, lv[L] the coarsest
     for (int l = 1; l < L; ++l) {
         bottom_restrict(A.lv[l - 1], A.P[l - 1], A.lv[l], A.P[l]);
@@ -977,7 +945,7 @@ int launch_vcycle_bottom(const Level *lv, int first, int nl, const double *aug, 
     attr[0].val.cooperative = 1;
     cfg.gridDim = dim3((unsigned)nblk);
     cfg.blockDim = dim3(BOT_T);
-    cfg.dynamicSmemBytes = sizeof(double) * (size_t)A.ndof;
+    cfg.dynamicSmemBytes = coarsest_smem(A.ndof);
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -993,7 +961,7 @@ int vcycle_bottom_blocks(int num_sms, int ndof, bool f32) {
     int per = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per, f32 ? (const void *)k_vcycle_bottom<true> : (const void *)k_vcycle_bottom<false>, BOT_T,
-        sizeof(double) * (size_t)ndof);
+        coarsest_smem(ndof));
     if (e != cudaSuccess || per < 1) return 0;
     return num_sms;  // one CTA per SM: the fewest arrivals per barrier
 }

@@ -18,8 +18,8 @@
 //   restrict_stencil_aos_kernel_1 (grid_ex.cu:1065-1160): deeper levels R A P
 //     from the FP16 finer stencil.
 //   solveHostEquation / assembleHostMatrix (grid.cpp:349-424): coarsest level.
-//     Replaced by a dense FP64 inverse built on the device (Gauss-Jordan with
-//     partial pivoting) and applied as a GEMV per load case.
+//     Replaced by a dense FP64 inverse built on the device (panel-wise Gauss-Jordan
+//     with partial pivoting) and applied to the six load cases at once.
 #include "h3d_internal.cuh"
 
 namespace h3d {
@@ -317,186 +317,270 @@ void launch_galerkin(const Level &F, const Level &C, cudaStream_t s) {
 }
 
 // ---- coarsest level ---------------------------------------------------------------
-// aug: [n][2n] row-major, left = K over unique DOFs (3*lexid + comp), right = I.
-// One thread per row (vertex lex, component i) adds its 27 neighbour blocks in
-// neighbour order d = 0..26, so entries that several periodic images of one
-// neighbour fall on (grids of two or three cells per axis) are summed in a fixed
-// order and the coarsest inverse is the same from run to run.
+// Coarsest matrix K over the unique DOFs (3*lexid + comp), n x n row-major.  One
+// thread per (row, column vertex) adds the row vertex's neighbour blocks that fall
+// on the column vertex, in neighbour order d = 0..26 (several do only on grids of
+// two or three cells per axis), so the matrix is the same from run to run and is
+// written once, coalesced, without a clearing pass.
 template <bool F32>
-__global__ void k_coarse_assemble(Planes C, const uint4 *__restrict__ st, double *aug, int n) {
+__global__ void __launch_bounds__(256) k_coarse_assemble(Planes C, const uint4 *__restrict__ st, double *a, int n) {
+    const int nv = n / 3;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= C.nv * 3) return;
-    const long long lex = t / 3;
-    const int i = (int)(t % 3);
-    const int x = (int)(lex % C.n[0]);
-    const int y = (int)((lex / C.n[0]) % C.n[1]), z = (int)(lex / ((long long)C.n[0] * C.n[1]));
+    if (t >= (long long)n * nv) return;
+    const int w = (int)(t % nv), row = (int)(t / nv), i = row % 3, lex = row / 3;
+    const int n0 = C.n[0], n1 = C.n[1], n2 = C.n[2];
+    const int x = lex % n0, y = lex / n0 % n1, z = lex / (n0 * n1);
+    const int wx = w % n0, wy = w / n0 % n1, wz = w / (n0 * n1);
     const long long v = vidx(C, x, y, z);
-    double *row = aug + (3 * lex + i) * (2LL * n);
-    for (int d = 0; d < 27; d++) {
-        const int wx = wrap(x + d % 3 - 1, C.n[0]), wy = wrap(y + d / 3 % 3 - 1, C.n[1]), wz = wrap(z + d / 9 - 1, C.n[2]);
-        const long long w = wx + (long long)C.n[0] * (wy + (long long)C.n[1] * wz);
-        for (int j = 0; j < 3; j++) row[3 * w + j] += (double)StencilStore<F32>::get(st, C.nv, v, 9 * d + 3 * i + j);
-    }
-    row[n + 3 * lex + i] = 1.0;
-}
-
-void launch_coarse_assemble(const Level &C, double *aug, cudaStream_t s) {
-    const int n = (int)(3 * C.P.nv);
-    cudaMemsetAsync(aug, 0, sizeof(double) * (size_t)n * 2 * n, s);
-    const long long nt = C.P.nv * 3;
-    if (C.st32) k_coarse_assemble<true><<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(C.P, C.st, aug, n);
-    else k_coarse_assemble<false><<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(C.P, C.st, aug, n);
-}
-
-// Gauss-Jordan elimination with partial pivoting on [K | I] (n rows, 2n columns,
-// FP64; grid.cpp:385-424 inverts the same matrix on the host).  One launch per
-// pivot column spreads the rank-1 update over every SM; the pivot search, row
-// swap and scaling of the next column are done by whichever CTA of a launch
-// finishes last (an arrival counter, no waiting), so a factorisation is n + 1
-// launches.  Scratch behind the matrix: the n elimination factors of the current
-// column and the arrival counter.
-constexpr int GJ_THREADS = 256;
-constexpr int GJ_TC = 64;                          // tile columns (lanes of a row)
-constexpr int GJ_RPT = 8;                          // rows per thread
-constexpr int GJ_TR = GJ_RPT * GJ_THREADS / GJ_TC; // tile rows
-
-// pivot step of column k by one CTA: the row among k..n-1 with the largest |a_ik|
-// (ties: the lowest row) swapped into row k and scaled by 1 / a_kk; col_i = a_ik
-// (0 for the pivot row) for the elimination launch of column k
-__device__ void gj_pivot(double *a, int n, int k, double *col, int *flag) {
-    __shared__ double rmax[GJ_THREADS / 32];
-    __shared__ int ridx[GJ_THREADS / 32];
-    __shared__ int piv;
-    const int tid = threadIdx.x, m = 2 * n;
-    double best = -1.0;
-    int bi = k;
-    for (int i = k + tid; i < n; i += GJ_THREADS) {
-        const double v = fabs(__ldcg(&a[(long long)i * m + k]));
-        if (v > best) { best = v; bi = i; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_down_sync(0xffffffffu, best, o);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    if ((tid & 31) == 0) { rmax[tid >> 5] = best; ridx[tid >> 5] = bi; }
-    __syncthreads();
-    if (tid == 0) {
-        double b = -1.0;
-        int p = k;
-        for (int w = 0; w < GJ_THREADS / 32; w++)
-            if (rmax[w] > b || (rmax[w] == b && ridx[w] < p)) { b = rmax[w]; p = ridx[w]; }
-        piv = p;
-        if (!(b > 0.0)) *flag = 1;
-    }
-    __syncthreads();
-    const int p = piv;
-    if (p != k)
-        for (int j = k + tid; j < m; j += GJ_THREADS) {
-            const double t = __ldcg(&a[(long long)k * m + j]);
-            a[(long long)k * m + j] = __ldcg(&a[(long long)p * m + j]);
-            a[(long long)p * m + j] = t;
-        }
-    __syncthreads();
-    const double inv = 1.0 / __ldcg(&a[(long long)k * m + k]);
-    __syncthreads();
-    for (int j = k + tid; j < m; j += GJ_THREADS) a[(long long)k * m + j] = __ldcg(&a[(long long)k * m + j]) * inv;
-    for (int i = tid; i < n; i += GJ_THREADS) col[i] = (i == k) ? 0.0 : __ldcg(&a[(long long)i * m + k]);
-}
-
-__global__ void __launch_bounds__(GJ_THREADS) k_gj_first(double *a, int n, double *col, int *flag) {
-    gj_pivot(a, n, 0, col, flag);
-}
-
-// elimination of column k from every other row over columns k..2n-1
-// (a_ij -= col_i a_kj), then the pivot step of column k + 1 by the last CTA
-__global__ void __launch_bounds__(GJ_THREADS) k_gj_step(double *a, int n, int k, double *col, int *flag,
-                                                        unsigned *arrived) {
-    const int m = 2 * n;
-    const int j = k + blockIdx.x * GJ_TC + (threadIdx.x % GJ_TC);
-    const int i0 = blockIdx.y * GJ_TR + threadIdx.x / GJ_TC;
-    if (j < m) {
-        const double akj = __ldcg(&a[(long long)k * m + j]);
-#pragma unroll
-        for (int r = 0; r < GJ_RPT; ++r) {
-            const int i = i0 + r * (GJ_THREADS / GJ_TC);
-            if (i < n && i != k) {
-                double *e = &a[(long long)i * m + j];
-                *e = fma(-__ldcg(&col[i]), akj, __ldcg(e));
+    double s[3] = {0, 0, 0};
+    for (int dz = -1; dz <= 1; dz++) {
+        if (wrap(z + dz, n2) != wz) continue;
+        for (int dy = -1; dy <= 1; dy++) {
+            if (wrap(y + dy, n1) != wy) continue;
+            for (int dx = -1; dx <= 1; dx++) {
+                if (wrap(x + dx, n0) != wx) continue;
+                const int d = 9 * (dz + 1) + 3 * (dy + 1) + dx + 1;
+                for (int j = 0; j < 3; j++) s[j] += (double)StencilStore<F32>::get(st, C.nv, v, 9 * d + 3 * i + j);
             }
         }
     }
-    if (k + 1 >= n) return;
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(arrived, 1u) == gridDim.x * gridDim.y - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    gj_pivot(a, n, k + 1, col, flag);
-    if (threadIdx.x == 0) *arrived = 0u;
+    double *o = a + (long long)row * n + 3 * w;
+    for (int j = 0; j < 3; j++) o[j] = s[j];
 }
 
-size_t gauss_jordan_doubles(int n) { return (size_t)n * 2 * n + n + 1; }
+// Coarsest inverse: in-place Gauss-Jordan elimination with partial pivoting in FP64
+// (grid.cpp:385-424 inverts the same matrix on the host), NB pivot columns (a panel)
+// per launch.  The elimination of a panel, row swaps included, is T = I outside the
+// panel's columns and the n x NB matrix G in them, so every other column becomes
+//   x_i <- (i in the panel's rows ? 0 : x_i) + sum_j G_ij x_{k+j}   (rows after the swaps)
+// and the panel's own columns become G.  Launch k applies panel k to all columns
+// (32 columns per warp, one per lane, the NB pivot-row values of a column in
+// registers), while its first CTA applies it to panel k + 1's columns alone and
+// factors that panel at once: one row per thread (R rows for the large sizes), the
+// panel in registers, two barriers per pivot.  The matrix goes back and forth
+// between two buffers, so the row swaps are an index map (srow) on the reads; the
+// last launch also undoes them on the columns, which leaves K^-1.
+// The factorisation is a serial chain of n pivot steps, bound by their latency: one
+// launch per pivot column over [K | I] took 7.3 us a step (1.41 ms for 192 unknowns,
+// 5.9 ms for 648); here a panel's steps stay inside one CTA.
+// The pivot is the largest |a_ij| to 20 mantissa bits, the first of equals.
+constexpr int GJ_ROWS_PER_WARP = 4;  // rows of a tile per warp
+
+struct GjArgs {
+    const double *src;   // the matrix before panel k
+    double *dst;         // after it
+    const double *G;     // panel k's G (n x NB, rows after its swaps, zero padded)
+    double *Gn;          // panel k + 1's
+    const int *srow;     // row of src that holds row i after panel k's swaps
+    int *srown;          // the same for panel k + 1
+    const int *orow;     // row of K that row i holds after panel k's swaps
+    int *orown;
+    int *flag;
+    int n, k, np;        // k = -1: factor panel 0 only; k = np - 1: apply the last panel
+};
+
+template <int NB, int R, int MAXT>
+__global__ void __launch_bounds__(MAXT) k_gj_panel(GjArgs g) {
+    const int n = g.n, k = g.k, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    const int c0 = k * NB, cn = c0 + NB;  // first column of panel k, of panel k + 1
+    const bool has_next = k + 1 < g.np;
+    if (!has_next || blockIdx.x > 0) {
+        // apply panel k to a tile of 32 columns
+        const int ncol = (n + 31) / 32, t = (int)blockIdx.x - (has_next ? 1 : 0);
+        const int rb = GJ_ROWS_PER_WARP * nw, r0 = (t / ncol) * rb, r1 = min(n, r0 + rb);
+        const int c = (t % ncol) * 32 + lane;
+        const bool own = c >= c0 && c < cn, skip = c >= n || (has_next && c >= cn && c < cn + NB);
+        double x[NB];
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+            x[j] = (skip || own || c0 + j >= n) ? 0.0 : __ldg(&g.src[(long long)__ldg(&g.srow[c0 + j]) * n + c]);
+        const int cd = skip ? 0 : (has_next ? c : __ldg(&g.orow[c]));
+        for (int i = r0 + wid; i < r1; i += nw) {
+            const double *Gi = g.G + (long long)i * NB;
+            double v = (skip || own || (i >= c0 && i < cn)) ? 0.0 : __ldg(&g.src[(long long)__ldg(&g.srow[i]) * n + c]);
+#pragma unroll
+            for (int j = 0; j < NB; ++j) v = fma(__ldg(Gi + j), x[j], v);
+            if (own) v = __ldg(Gi + (c - c0));
+            if (!skip) g.dst[(long long)i * n + cd] = v;
+        }
+        return;
+    }
+    // panel k + 1: apply panel k to its columns, then factor it
+    extern __shared__ int srow_s[];  // n: rows of dst after this panel's swaps
+    __shared__ double xs[NB][NB];
+    __shared__ double rowp[2][NB], rowq[2][NB];
+    __shared__ unsigned keys[2][32];
+    __shared__ int krow[2][32];
+    const int nbn = min(NB, n - cn);
+    for (int i = tid; i < n; i += blockDim.x) srow_s[i] = i;
+    double a[R][NB];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = tid + r * (int)blockDim.x;
+        const bool in = i < n, pan = k >= 0 && i >= c0 && i < cn;
+        const int si = in ? (k >= 0 ? __ldg(&g.srow[i]) : i) : 0;
+#pragma unroll
+        for (int c = 0; c < NB; ++c) a[r][c] = (in && !pan && c < nbn) ? __ldg(&g.src[(long long)si * n + cn + c]) : 0.0;
+    }
+    if (k >= 0) {
+        for (int q = tid; q < NB * NB; q += blockDim.x) {
+            const int j = q / NB, c = q % NB;
+            xs[j][c] = c < nbn ? __ldg(&g.src[(long long)__ldg(&g.srow[c0 + j]) * n + cn + c]) : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = tid + r * (int)blockDim.x;
+            const double *Gi = g.G + (long long)(i < n ? i : 0) * NB;
+#pragma unroll 4
+            for (int j = 0; j < NB; ++j) {
+                const double gj = __ldg(Gi + j);
+#pragma unroll
+                for (int c = 0; c < NB; ++c) a[r][c] = fma(gj, xs[j][c], a[r][c]);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+        if (j >= nbn) break;
+        const int q = cn + j, b = j & 1;  // pivot row; buffer of this step
+        unsigned key = 0;                 // 0: not a candidate
+        int kr = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = tid + r * (int)blockDim.x;
+            const unsigned kk = (i >= q && i < n) ? ((unsigned)__double2hiint(a[r][j]) & 0x7fffffffu) + 1u : 0u;
+            if (kk > key) { key = kk; kr = i; }
+        }
+        const unsigned wm = __reduce_max_sync(0xffffffffu, key);
+        const unsigned who = __ballot_sync(0xffffffffu, key == wm);
+        if (lane == __ffs(who) - 1) { keys[b][wid] = wm; krow[b][wid] = kr; }
+        __syncthreads();
+        const unsigned wk = lane < nw ? keys[b][lane] : 0u;
+        const unsigned bm = __reduce_max_sync(0xffffffffu, wk);
+        const int p = krow[b][__ffs(__ballot_sync(0xffffffffu, wk == bm)) - 1];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = tid + r * (int)blockDim.x;
+            if (i == p)
+#pragma unroll
+                for (int c = 0; c < NB; ++c) rowp[b][c] = a[r][c];
+            if (i == q)
+#pragma unroll
+                for (int c = 0; c < NB; ++c) rowq[b][c] = a[r][c];
+        }
+        __syncthreads();
+        const double piv = rowp[b][j], inv = 1.0 / piv;
+        if (tid == 0) {
+            if (!(fabs(piv) > 0.0)) *g.flag = 1;
+            const int t = srow_s[p];
+            srow_s[p] = srow_s[q];
+            srow_s[q] = t;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = tid + r * (int)blockDim.x;
+            if (i == p && p != q)  // the row swapped out of the pivot position
+#pragma unroll
+                for (int c = 0; c < NB; ++c) a[r][c] = rowq[b][c];
+            if (i == q) {
+#pragma unroll
+                for (int c = 0; c < NB; ++c) a[r][c] = c == j ? inv : rowp[b][c] * inv;
+            } else {
+                const double f = -(a[r][j] * inv);
+#pragma unroll
+                for (int c = 0; c < NB; ++c) a[r][c] = c == j ? f : fma(f, rowp[b][c], a[r][c]);
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = tid + r * (int)blockDim.x;
+        if (i >= n) continue;
+        g.srown[i] = srow_s[i];
+        g.orown[i] = k >= 0 ? __ldg(&g.orow[srow_s[i]]) : srow_s[i];
+#pragma unroll
+        for (int c = 0; c < NB; ++c) g.Gn[(long long)i * NB + c] = c < nbn ? a[r][c] : 0.0;
+    }
+}
+
+// panel width, rows per thread and thread limit by size: a panel row is 2 NB
+// registers, so 16 columns fit up to 1024 one-row threads (coarsest grids to 6 x 7 x 8
+// vertices), and 8 columns with two rows per thread hold the rest (7^3: 1029 unknowns
+// to 8^3: 1536)
+static int gj_width(int n) { return n <= 1024 ? 16 : 8; }
+static int gj_panels(int n) { return (n + gj_width(n) - 1) / gj_width(n); }
+
+// [K^-1 | the other buffer | two G | two srow, two orow]
+size_t gauss_jordan_doubles(int n) { return (size_t)n * n * 2 + (size_t)n * 16 * 2 + (size_t)n * 2 + 2; }
+
+// K is assembled into the buffer from which the panels' alternation ends in the first
+static double *gj_start(double *aug, int n) { return aug + (gj_panels(n) & 1 ? (size_t)n * n : 0); }
+
+void launch_coarse_assemble(const Level &C, double *aug, cudaStream_t s) {
+    const int n = (int)(3 * C.P.nv);
+    const long long nt = (long long)n * C.P.nv;
+    double *a = gj_start(aug, n);
+    if (C.st32) k_coarse_assemble<true><<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(C.P, C.st, a, n);
+    else k_coarse_assemble<false><<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(C.P, C.st, a, n);
+}
+
+template <int NB, int R, int MAXT>
+static void gj_run(double *aug, int n, int *flag, cudaStream_t s) {
+    const int np = gj_panels(n);
+    const unsigned nt = (unsigned)(((n + R - 1) / R + 31) / 32 * 32);
+    const unsigned rb = GJ_ROWS_PER_WARP * (nt / 32);
+    const unsigned tiles = (unsigned)((n + 31) / 32) * ((n + rb - 1) / rb);
+    double *buf[2] = {aug, aug + (size_t)n * n};
+    double *G[2] = {buf[1] + (size_t)n * n, buf[1] + (size_t)n * n + (size_t)n * NB};
+    int *idx = reinterpret_cast<int *>(buf[1] + (size_t)n * n + (size_t)n * 16 * 2);
+    int *srow[2] = {idx, idx + n}, *orow[2] = {idx + 2 * n, idx + 3 * n};
+    for (int k = -1; k < np; k++) {
+        GjArgs g;
+        const int from = (np + (k < 0 ? 0 : k)) & 1, cur = k & 1, next = (k + 1) & 1;
+        g.src = buf[from];
+        g.dst = buf[from ^ 1];
+        g.G = G[cur];
+        g.Gn = G[next];
+        g.srow = srow[cur];
+        g.srown = srow[next];
+        g.orow = orow[cur];
+        g.orown = orow[next];
+        g.flag = flag;
+        g.n = n;
+        g.k = k;
+        g.np = np;
+        const unsigned nb = k < 0 ? 1u : tiles + (k + 1 < np ? 1u : 0u);
+        k_gj_panel<NB, R, MAXT><<<nb, nt, sizeof(int) * (size_t)n, s>>>(g);
+    }
+}
 
 void launch_gauss_jordan(double *aug, int n, int *flag, cudaStream_t s) {
-    double *col = aug + (size_t)n * 2 * n;
-    unsigned *arrived = reinterpret_cast<unsigned *>(col + n);
-    cudaMemsetAsync(arrived, 0, sizeof(unsigned), s);
-    k_gj_first<<<1, GJ_THREADS, 0, s>>>(aug, n, col, flag);
-    const unsigned gy = (unsigned)((n + GJ_TR - 1) / GJ_TR);
-    for (int k = 0; k < n; k++) {
-        const unsigned gx = (unsigned)((2 * n - k + GJ_TC - 1) / GJ_TC);
-        k_gj_step<<<dim3(gx, gy), GJ_THREADS, 0, s>>>(aug, n, k, col, flag, arrived);
-    }
+    if (n <= 704) gj_run<16, 1, 704>(aug, n, flag, s);
+    else if (n <= 1024) gj_run<16, 1, 1024>(aug, n, flag, s);
+    else gj_run<8, 2, 768>(aug, n, flag, s);
 }
 
-// one block per load case c: b (optionally minus its mean per component), x = K^-1 b;
-// b: n doubles of shared memory
-__device__ __forceinline__ void coarse_apply_block(const Planes &C, const double *__restrict__ aug, int n, int project,
-                                                   const float *__restrict__ f, float *u, int c, double *b) {
-    __shared__ double mean[3];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const long long lex = i / 3;
-        const int comp = i % 3;
-        const int x = (int)(lex % C.n[0]), y = (int)((lex / C.n[0]) % C.n[1]), z = (int)(lex / ((long long)C.n[0] * C.n[1]));
-        b[i] = f[fidx(3 * c + comp, vidx(C, x, y, z))];
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double s = 0;
-        if (project)
-            for (int i = threadIdx.x; i < n; i += 3) s += b[i];
-        mean[threadIdx.x] = s / (double)(n / 3);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) b[i] -= mean[i % 3];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double *row = aug + (long long)i * 2 * n + n;
-        double s = 0;
-        for (int j = 0; j < n; j++) s = fma(row[j], b[j], s);
-        const long long lex = i / 3;
-        const int comp = i % 3;
-        const int x = (int)(lex % C.n[0]), y = (int)((lex / C.n[0]) % C.n[1]), z = (int)(lex / ((long long)C.n[0] * C.n[1]));
-        u[fidx(3 * c + comp, vidx(C, x, y, z))] = (float)s;
-    }
+// x = K^-1 b for the six load cases: one warp per row of K^-1 (coarsest_rows), all
+// cases from one read of the row.  One thread per row and one CTA per load case read
+// the rows with a stride of 2n doubles, six times: 23 us for 192 unknowns, 237 us for
+// 648.
+__global__ void __launch_bounds__(COARSEST_T) k_coarse_apply(Planes C, const double *__restrict__ inv, int n,
+                                                             int project, const float *__restrict__ f, float *u) {
+    extern __shared__ float b[];
+    coarsest_rows<false>(C, inv, n, project, f, u, b, blockIdx.x, gridDim.x);
 }
 
-__global__ void __launch_bounds__(256) k_coarse_apply(Planes C, const double *__restrict__ aug, int n, int project,
-                                                      const float *__restrict__ f, float *u) {
-    extern __shared__ double b[];
-    coarse_apply_block(C, aug, n, project, f, u, blockIdx.x, b);
-}
+static unsigned coarsest_blocks(int n) { return (unsigned)((n + COARSEST_T / 32 - 1) / (COARSEST_T / 32)); }
 
 void launch_coarse_apply(const Level &C, const double *aug, int project, cudaStream_t s) {
     const int n = (int)(3 * C.P.nv);
-    k_coarse_apply<<<NCASE, 256, (size_t)n * sizeof(double), s>>>(C.P, aug, n, project, C.f, C.u);
+    k_coarse_apply<<<coarsest_blocks(n), COARSEST_T, coarsest_smem(n), s>>>(C.P, aug, n, project, C.f, C.u);
 }
 
-// lockstep batches: the coarsest solves of several designs in one launch, six
-// CTAs (one per load case) per design, each the CTA of the design's own launch
+// lockstep batches: the coarsest solves of several designs in one launch, grid row y
+// for slot y; a slot's CTAs are those of the design's own launch
 struct CoarsestEnt {
     Planes C;
     const double *aug;
@@ -509,14 +593,15 @@ struct CoarsestBatchTab {
     CoarsestEnt e[BATCH_MAX];
 };
 
-__global__ void __launch_bounds__(256) k_coarse_apply_batch(const CoarsestBatchTab *__restrict__ t,
+__global__ void __launch_bounds__(COARSEST_T) k_coarse_apply_batch(const CoarsestBatchTab *__restrict__ t,
                                                             const int *__restrict__ active, int project) {
-    extern __shared__ double b[];
+    extern __shared__ float b[];
     __shared__ __align__(16) unsigned buf[sizeof(CoarsestEnt) / 4];
-    const int i = blockIdx.x / NCASE, c = blockIdx.x % NCASE;
+    const int i = blockIdx.y;
     if (!__ldg(&active[t->e[i].design])) return;
     const CoarsestEnt &e = stage_args(t->e[i], buf);
-    coarse_apply_block(e.C, e.aug, e.n, project, e.f, e.u, c, b);
+    const unsigned nb = (unsigned)((e.n + COARSEST_T / 32 - 1) / (COARSEST_T / 32));
+    if (blockIdx.x < nb) coarsest_rows<false>(e.C, e.aug, e.n, project, e.f, e.u, b, blockIdx.x, nb);
 }
 
 int coarsest_batch_create(const Level *const *lv, const double *const *aug, const int *design, int n, BatchTab *out) {
@@ -537,15 +622,11 @@ int coarsest_batch_create(const Level *const *lv, const double *const *aug, cons
     void *d = nullptr;
     int rc = cudaMalloc(&d, sizeof(CoarsestBatchTab)) == cudaSuccess ? 0 : -2;
     if (rc == 0 && cudaMemcpy(d, t, sizeof(CoarsestBatchTab), cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
-    if (rc == 0 && nmax * sizeof(double) + sizeof(CoarsestEnt) > 48 * 1024 &&
-        cudaFuncSetAttribute(k_coarse_apply_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(nmax * sizeof(double))) != cudaSuccess)
-        rc = -2;
     if (rc == 0) {
         out->dev = d;
         out->n = n;
-        out->grid[0] = (unsigned)(n * NCASE);
-        out->smem = (size_t)nmax * sizeof(double);
+        out->grid[0] = coarsest_blocks(nmax);
+        out->smem = coarsest_smem(nmax);
     } else if (d) {
         cudaFree(d);
     }
@@ -554,7 +635,7 @@ int coarsest_batch_create(const Level *const *lv, const double *const *aug, cons
 }
 
 void launch_coarse_apply_batch(const BatchTab &t, const int *active, int project, cudaStream_t s) {
-    k_coarse_apply_batch<<<t.grid[0], 256, t.smem, s>>>(static_cast<const CoarsestBatchTab *>(t.dev), active,
+    k_coarse_apply_batch<<<dim3(t.grid[0], (unsigned)t.n), COARSEST_T, t.smem, s>>>(static_cast<const CoarsestBatchTab *>(t.dev), active,
                                                          project);
 }
 
