@@ -181,16 +181,18 @@ def launches_per_step(nl, vcycles, reso, refine, refinements, coarsest_nv, mixed
     solutions, so the FP64 solution is cleared instead of copied and centred (no
     kernel for 3) and the first refinement step sets f from f0 (1 kernel) instead
     of u64 += u and the FP64 residual (2)"""
-    nblk = -(-(reso ** 3 // 8) // 128) * 3 * 8                  # fine residual norm partials
+    nblk = reso * reso                                          # fine residual norm partials, one per row
     finish = 2 if nblk > 4096 else 1                            # one- or two-stage norm reduction
-    fine = 8 + 1 + finish + 8                                   # GS (last colour with its residual), residual, norms, GS
+    fine = 4 + 1 + finish + 4                                   # GS (two colours per launch), residual, norms, GS
     if mixed:
-        fine = 8 + 1 + 1 + 8                                    # GS, tensor-core residual, norms, GS
+        fine = 4 + 1 + 1 + 4                                    # GS, tensor-core residual, norms, GS
     coarse = (nl - 2) * (8 + 1 + 8)                             # GS per colour, residual, GS per colour
     per_cycle = fine + coarse + 2 * (nl - 1) + 1 + 1            # restrict, prolong, coarsest apply, deflation
     per_refine = 1 + 1 + 2 + 3                                  # u64 += u, residual64, norms, deflation restart
-    setup = 1 + 1 + 1 + (nl - 2) + 1 + 1 + 3 * coarsest_nv      # density, level 1, pin patch, deeper, assemble,
-    #                                                             first pivot, one launch per pivot column
+    ndof = 3 * coarsest_nv
+    panels = -(-ndof // (16 if ndof <= 1024 else 8))
+    setup = 1 + 1 + 1 + (nl - 2) + 1 + 1 + panels               # density, level 1, pin patch, deeper, assemble,
+    #                                                             first panel, one launch per panel
     if refine:
         pre = 1 + 3 + 2                                         # rhs, balance, norms of f
         post = 2                                                # C: energies, reduction

@@ -1036,7 +1036,7 @@ int h3d_update_residual(h3d_handle *h, int level) {
             launch_fine_residual_tc(h->lv[0], h->rho, h->ke, nullptr, fine_residual_tc_blocks(h->lv[0].P, h->num_sms),
                                     h->d_tcflag, h->stream);
         } else {
-            launch_fine_residual(h->lv[0], h->rho, h->ke, nullptr, 0, h->stream);
+            launch_fine_residual(h->lv[0], h->rho, h->ke, nullptr, h->stream);
         }
     } else {
         if (!h->have_stencils) return fail(h, H3D_ERR_STATE, "no stencils");

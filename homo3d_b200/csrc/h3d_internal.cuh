@@ -292,13 +292,11 @@ struct StencilStore<true> {
 // ---- launch wrappers (kernels in the .cu files) --------------------------
 // fine level (k_fine.cu)
 void launch_fine_gs(const Level &L, const float *rho, const KeMat &ke, float w, cudaStream_t s);
-// a colour sweep followed by the level-0 residual and its norm partials (the last
-// colour's launch computes its own vertices' residual)
+// a colour sweep followed by the level-0 residual and its norm partials
 void launch_fine_gs_residual(const Level &L, const float *rho, const KeMat &ke, float w, double *norm_partial,
                              cudaStream_t s);
-void launch_fine_residual(const Level &L, const float *rho, const KeMat &ke, double *norm_partial,
-                          int nblk_norm, cudaStream_t s);
-// number of per-block norm partials launch_fine_residual writes
+void launch_fine_residual(const Level &L, const float *rho, const KeMat &ke, double *norm_partial, cudaStream_t s);
+// number of norm partials (rows of six) launch_fine_residual writes
 int fine_residual_blocks(const Level &L);
 void launch_rhs(const Level &L, const float *rho, const RhsTab &g, float *f, cudaStream_t s);
 // r = f - K u with u in FP64, the operator in difference form (refined precision)
@@ -422,8 +420,8 @@ void launch_warmnet_to_chi(const Planes &P, const float *y, int R, double *chi, 
 // copy a table to the device (not inside a stream capture) and return 0, -1 for a
 // slot count outside 1..BATCH_MAX, -2 if the device table cannot be allocated.
 // design[i]: slot i's index in the `active` flags the launches read.
-// level 0 of each design: the sweep (launch shape 0: six cases per thread, 1: three),
-// the seven-colour residual and the deflation (state: the design's deflation
+// level 0 of each design: the sweep (launch shape 0: three cases per thread, 1: two),
+// the residual and the deflation (state: the design's deflation
 // state); scratch: the sweeps iterate on each design's r instead of u (timing)
 int fine_batch_create(const Level *const *lv0, const float *const *rho, double *const *partial,
                       double *const *state, const int *design, int n, bool scratch, BatchTab *out);

@@ -13,27 +13,31 @@
 //
 // B200 design.  The element loop is reorganised per neighbour: for each of the 26
 // neighbours the 3x3 coupling block sum_e rho_e Ke[a_e][b_e] is formed once (Ke
-// entries are compile-time offsets into the kernel-parameter bank, so they are
-// FFMA operands) and applied to the load cases, two cases at a time as packed
-// FP32x2 lane pairs.  The colour sweep serves each vertex by one thread with all
-// six cases (the block is built once per vertex; the sweep is bound by instruction
-// issue, 128 registers, 4 CTAs/SM); the residuals serve it by three threads with
-// two cases each in adjacent CTAs (fewer registers: the residual also writes r and
-// reduces the norms), where the densities and neighbour rows the three share hit
-// L1/L2, and all eight colours of a residual go in one launch (seven in a V-cycle,
-// where the sweep's last colour launch writes colour 7's residual).  The operator is
-// applied in difference form, sum_{d != 0} A_d (u_{v+d} - u_v), and the
-// Gauss-Seidel step as u += D^-1 r with
+// entries are compile-time offsets into the kernel-parameter bank) and applied to a
+// thread's load cases.  A thread serves the two vertices x = 2i + 1 and x = 2i of a
+// row, as the two lanes of packed FP32x2 values: the 27 neighbours of both lie in nine
+// rows, and each row gives both from four values per plane instead of six.  A sweep's
+// launch takes the rows of one (y, z) parity, i.e. two of the eight colours: the odd
+// vertices are updated first, the even ones after a barrier (a CTA holds whole rows, so
+// the periodic neighbour in x is in the CTA); see k_fine_gs.  The residual runs all
+// rows in one launch.  The operator is applied in difference form,
+// sum_{d != 0} A_d (u_{v+d} - u_v), and the Gauss-Seidel step as u += D^-1 r with
 // the components in the reference's order: the same iteration in exact
-// arithmetic, and in FP32 it keeps rigid translations exact (see fine_apply).
+// arithmetic, and in FP32 it keeps rigid translations exact (see pair_rows).
 #include <type_traits>
 
 #include "h3d_internal.cuh"
 
 namespace h3d {
 
-constexpr int CPT = 2;            // load cases per thread of the FP32 residual (three threads per vertex)
-constexpr int RES_MINB = 6;       // its CTAs per SM
+constexpr int CPT = 2;            // load cases per thread of the FP32 residual
+constexpr int RES_MINB = 4;       // its CTAs of 128 threads per SM
+// Row blocks between a CTA of the pair kernels and the one whose rows it brings into L2.
+// Both kernels wait on loads with few warps (128 registers: 4 CTAs/SM), and more than
+// half of their L1 misses went on to DRAM.  Measured at 256^3: the sweep 2.60 ms without
+// prefetch, 2.36 / 2.32 / 2.29 / 2.29 ms at 150 / 100 / 50 / 20 row blocks, the residual
+// 2.72 ms without, 2.60 / 2.51 / 2.50 / 2.47 at 150 / 50 / 25 / 10.
+constexpr unsigned GS_AHEAD = 20, RES_AHEAD = 10;
 constexpr int CPT64 = 2;          // load cases per thread of the FP64-solution residual
 constexpr int MINB64 = 4;         // its CTAs per SM
 constexpr int FBS = 128;          // threads per CTA
@@ -49,6 +53,7 @@ struct FineArgs {
     long long P;   // vertices per colour plane
     float w;
     FastDiv dh0, dh1;  // division by h[0], h[1]
+    int rows;          // whole rows per CTA of the pair kernels (pair_shape)
 };
 
 __device__ __forceinline__ void axis_nbrs(int i, int p, int h, int &im, int &ip) {
@@ -74,6 +79,62 @@ __host__ __device__ constexpr int first_shared(int d) {
         if (bx >= 0 && bx <= 1 && by >= 0 && by <= 1 && bz >= 0 && bz <= 1) return w;
     }
     return -1;
+}
+
+// one value, or the same quantity of the two vertices of a pair
+__device__ __forceinline__ float vadd(float a, float b) { return a + b; }
+__device__ __forceinline__ float vsub(float a, float b) { return a - b; }
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ void vzero(float &a) { a = 0.f; }
+__device__ __forceinline__ void vzero(double &a) { a = 0.0; }
+__device__ __forceinline__ void vzero(float2 &a) { a = make_float2(0.f, 0.f); }
+
+// The signed sums cs[m] of the densities rw over the elements shared with neighbour
+// (dx, dy, dz), folded one free axis at a time:
+// element pairs along the first free axis (their sum and difference), then
+// pairs of those along the next.  Along a free axis a the element with bit a
+// set enters with a minus sign when a lies in the mask m, so the sign of an
+// element is the parity of the mask axes on which it differs from w0.
+// 0 / 2 / 8 / 16 additions for a corner / edge / face neighbour / the vertex
+// itself, where the element-by-element sums took 4 / 8 / 16 / 32.
+template <typename T>
+__device__ __forceinline__ void fold_signed(const T rw[8], int dx, int dy, int dz, int w0, T cs[8]) {
+    int fa[3], nf = 0;  // the free axes (offset 0), ascending
+    if (dx == 0) fa[nf++] = 0;
+    if (dy == 0) fa[nf++] = 1;
+    if (dz == 0) fa[nf++] = 2;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        if (m != 0 && m != 3 && m != 5 && m != 6) { vzero(cs[m]); continue; }
+        if (nf == 0) {
+            cs[m] = rw[w0];
+        } else {
+            const int a = fa[0];
+            // level 1: pairs (w, w | a) for the 2^(nf-1) settings of the other free axes
+            T v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k >= (1 << (nf - 1))) continue;
+                int w = w0;
+                if (nf > 1 && (k & 1)) w |= 1 << fa[1];
+                if (nf > 2 && (k & 2)) w |= 1 << fa[2];
+                v[k] = ((m >> a) & 1) ? vsub(rw[w], rw[w | (1 << a)]) : vadd(rw[w], rw[w | (1 << a)]);
+            }
+            if (nf >= 2) {  // level 2: along fa[1]
+                const bool mb = (m >> fa[1]) & 1;
+                v[0] = mb ? vsub(v[0], v[1]) : vadd(v[0], v[1]);
+                if (nf == 3) v[2] = mb ? vsub(v[2], v[3]) : vadd(v[2], v[3]);
+            }
+            if (nf == 3) {  // level 3: along fa[2]
+                const bool mc = (m >> fa[2]) & 1;
+                v[0] = mc ? vsub(v[0], v[2]) : vadd(v[0], v[2]);
+            }
+            cs[m] = v[0];
+        }
+    }
 }
 
 // geometry of one colour-K vertex: its element densities and the offsets of its
@@ -130,50 +191,12 @@ struct VertexGeo {
 #pragma unroll
             for (int c = 0; c < 3; ++c) A[3 * r + c] = kk[(3 * an + r) * 24 + 3 * bn + c] * cs[(1 << r) ^ (1 << c)];
     }
-    // The signed sums over the shared elements, folded one free axis at a time:
-    // element pairs along the first free axis (their sum and difference), then
-    // pairs of those along the next.  Along a free axis a the element with bit a
-    // set enters with a minus sign when a lies in the mask m, so the sign of an
-    // element is the parity of the mask axes on which it differs from w0.
-    // 0 / 2 / 8 / 16 additions for a corner / edge / face neighbour / the vertex
-    // itself, where the element-by-element sums took 4 / 8 / 16 / 32.
-    template <typename T>
-    __device__ __forceinline__ T rwv(int w) const { return (T)rw[w]; }
     template <typename T>
     __device__ __forceinline__ void signed_sums(int dx, int dy, int dz, int w0, T cs[8]) const {
-        int fa[3], nf = 0;  // the free axes (offset 0), ascending
-        if (dx == 0) fa[nf++] = 0;
-        if (dy == 0) fa[nf++] = 1;
-        if (dz == 0) fa[nf++] = 2;
+        T v[8];
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            if (m != 0 && m != 3 && m != 5 && m != 6) { cs[m] = T(0); continue; }
-            if (nf == 0) {
-                cs[m] = rwv<T>(w0);
-            } else {
-                const int a = fa[0];
-                // level 1: pairs (w, w | a) for the 2^(nf-1) settings of the other free axes
-                T v[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (k >= (1 << (nf - 1))) continue;
-                    int w = w0;
-                    if (nf > 1 && (k & 1)) w |= 1 << fa[1];
-                    if (nf > 2 && (k & 2)) w |= 1 << fa[2];
-                    v[k] = ((m >> a) & 1) ? rwv<T>(w) - rwv<T>(w | (1 << a)) : rwv<T>(w) + rwv<T>(w | (1 << a));
-                }
-                if (nf >= 2) {  // level 2: along fa[1]
-                    const bool mb = (m >> fa[1]) & 1;
-                    v[0] = mb ? v[0] - v[1] : v[0] + v[1];
-                    if (nf == 3) v[2] = mb ? v[2] - v[3] : v[2] + v[3];
-                }
-                if (nf == 3) {  // level 3: along fa[2]
-                    const bool mc = (m >> fa[2]) & 1;
-                    v[0] = mc ? v[0] - v[2] : v[0] + v[2];
-                }
-                cs[m] = v[0];
-            }
-        }
+        for (int w = 0; w < 8; ++w) v[w] = (T)rw[w];
+        fold_signed<T>(v, dx, dy, dz, w0, cs);
     }
     __device__ __forceinline__ void block(const KeMat &ke, int d, float A[9]) const { block_t<float>(ke.k, d, A); }
     // the coupling block in FP64 from an FP64 element matrix (the exact refinement
@@ -191,288 +214,435 @@ struct VertexGeo {
     }
 };
 
-// acc[3c+r] (c < CPT, cases cb..cb+CPT-1) = (K u)_v in difference form,
-// sum over the 26 neighbours of A_d (u_{v+d} - u_v), with u at the pinned origin
-// counted as 0.  Equal to sum_d A_d u_{v+d} in exact arithmetic (the blocks of a
-// row sum to zero), and exact for rigid translations in FP32 too, so the FP32
-// operator agrees with the FP64 difference-form residual of the refined mode on
-// the near-null translation mode of the pinned problem.
-template <int K, int C>
-__device__ __forceinline__ void fine_apply(const FineArgs &a, const KeMat &ke, const VertexGeo<K> &g, int cb,
-                                           const float uv[3 * C], float acc[3 * C]) {
-    constexpr int NP = C / 2;  // case pairs per thread
-    constexpr int NS = C % 2;  // an odd last case, on scalar lanes
-    // lane pair (case cb+2j, case cb+2j+1) of each component: Blackwell's packed
-    // FP32x2 add and FMA do both cases in one instruction with the rounding of the
-    // scalar forms, so the sums are the same as the scalar per-case loop (the odd
-    // case runs the scalar forms in the same order)
-    float2 acc2[3 * NP + 1], nuv2[3 * NP + 1];
-    float acc1[3 * NS + 1], nuv1[3 * NS + 1];
-#pragma unroll
-    for (int j = 0; j < NP; ++j)
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            acc2[3 * j + m] = make_float2(0.f, 0.f);
-            nuv2[3 * j + m] = make_float2(-uv[6 * j + m], -uv[6 * j + 3 + m]);
+// what a thread reads for a vertex whose values count as 0 (the pinned origin)
+__device__ float zero_planes[NF * FVB];
+
+// fidx(0, v) for v < 2^32
+__device__ __forceinline__ size_t fpos(unsigned v) { return (size_t)v + (size_t)(v >> 7) * ((NF - 1) * FVB); }
+
+// bring a vertex range of a field (72 bytes a vertex, all planes) into L2
+__device__ __forceinline__ void prefetch_field(const float *f, unsigned long long v0, unsigned long long v1) {
+    const unsigned long long b0 = v0 * (NF * 4) & ~15ull, b1 = v1 * (NF * 4) & ~15ull;
+    if (b1 > b0)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global((const char *)f + b0)),
+                     "r"((unsigned)(b1 - b0)));
+}
+
+// ---- vertex pairs --------------------------------------------------------------
+// Rows of a CTA of at most `tmax` threads: whole rows of h0 pairs, `rows` of them, on
+// rows * h0 of its threads (a multiple of 32), chosen to leave the fewest threads idle.
+struct PairShape {
+    int rows, threads;
+};
+static PairShape pair_shape(int h0) {
+    PairShape best = {1, (h0 + 31) / 32 * 32};
+    auto use = [&](const PairShape &s) { return (double)s.rows * h0 / s.threads; };
+    // up to 128 threads; up to 256 where that leaves more than 1 in 8 idle
+    for (int lim = 128; lim <= 256; lim *= 2) {
+        for (int r = 1; r * h0 <= lim; ++r) {
+            const PairShape s = {r, (r * h0 + 31) / 32 * 32};
+            if (use(s) > use(best) + 1e-9 || (use(s) > use(best) - 1e-9 && s.threads > best.threads))
+                best = s;
         }
-#pragma unroll
-    for (int m = 0; m < 3 * NS; ++m) {
-        acc1[m] = 0.f;
-        nuv1[m] = -uv[6 * NP + m];
+        if (use(best) >= 0.875) break;
     }
+    return best;
+}
+
+// The pair (x = 2i + 1, x = 2i) of row (j, l) of the rows with colours K0 (odd x) and
+// K0 + 1 (even x); lane x of every packed value is the odd vertex.
+struct PairGeo {
+    int K0;              // 0, 2, 4 or 6: the row's parities
+    float2 rw[8];        // element densities
+    int i, im, ip;       // pair index and its neighbours (periodic)
+    unsigned Y[3], Z[3]; // plane offsets of the neighbour rows
+    __device__ __forceinline__ PairGeo(const FineArgs &a, int k0, int ii, int j, int l) : K0(k0), i(ii) {
+        const int py = ((K0 >> 1) & 1) ^ 1, pz = ((K0 >> 2) & 1) ^ 1;
+        im = i == 0 ? a.h[0] - 1 : i - 1;
+        ip = i + 1 == a.h[0] ? 0 : i + 1;
+        const int y = 2 * j + py, z = 2 * l + pz;
+        const unsigned n0 = (unsigned)a.n[0], n01 = n0 * (unsigned)a.n[1];
+        const unsigned ye0 = (unsigned)(y == 0 ? a.n[1] - 1 : y - 1), ze0 = (unsigned)(z == 0 ? a.n[2] - 1 : z - 1);
+        const unsigned xe = 2u * (unsigned)i, xm = i == 0 ? n0 - 1 : xe - 1;
 #pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        if (d == 13) continue;
-        int Kn;
-        bool pinned;
-        const unsigned nid = g.nbr(a, d, Kn, pinned);
-        float A[9];
-        g.block(ke, d, A);
-        const float *up = a.u + fidx(3 * cb, nid);  // planes 3cb.. of the neighbour, FVB apart
+        for (int t = 0; t < 4; ++t) {
+            const float *row = a.rho + (n0 * ((t & 1) ? (unsigned)y : ye0) + n01 * ((t >> 1) ? (unsigned)z : ze0));
+            const float em = RHO_PENAL_MIN + __ldg(row + xm), e0 = RHO_PENAL_MIN + __ldg(row + xe),
+                        e1 = RHO_PENAL_MIN + __ldg(row + xe + 1);
+            rw[2 * t] = make_float2(e0, em);
+            rw[2 * t + 1] = make_float2(e1, e0);
+        }
+        int jm, jp, lm, lp;
+        axis_nbrs(j, py, a.h[1], jm, jp);
+        axis_nbrs(l, pz, a.h[2], lm, lp);
+        const unsigned h0 = (unsigned)a.h[0], h01 = h0 * (unsigned)a.h[1];
+        Y[0] = h0 * (unsigned)jm; Y[1] = h0 * (unsigned)j; Y[2] = h0 * (unsigned)jp;
+        Z[0] = h01 * (unsigned)lm; Z[1] = h01 * (unsigned)l; Z[2] = h01 * (unsigned)lp;
+    }
+    // coupling blocks of neighbour d of both vertices (VertexGeo::block_t)
+    __device__ __forceinline__ void block(const KeMat &ke, int d, float2 A[9]) const {
+        const int dx = d % 3 - 1, dy = d / 3 % 3 - 1, dz = d / 9 - 1;
+        const int w0 = first_shared(d);
+        float2 cs[8];
+        fold_signed<float2>(rw, dx, dy, dz, w0, cs);
+        const int an = 7 - w0;
+        const int bn = (1 - (w0 & 1) + dx) + 2 * (1 - ((w0 >> 1) & 1) + dy) + 4 * (1 - (w0 >> 2) + dz);
 #pragma unroll
-        for (int j = 0; j < NP; ++j) {
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float k = ke.k[(3 * an + r) * 24 + 3 * bn + c];
+                const float2 v = cs[(1 << r) ^ (1 << c)];
+                A[3 * r + c] = make_float2(k * v.x, k * v.y);
+            }
+    }
+    // first index of row (dy, dz) in its odd vertices' colour plane (the even ones: + P);
+    // its first even vertex is the pinned origin if `origin`
+    __device__ __forceinline__ unsigned row(const FineArgs &a, int dy, int dz, bool &origin) const {
+        const unsigned off = Y[dy + 1] + Z[dz + 1];
+        const int Kn = K0 ^ (((dy & 1) << 1) | ((dz & 1) << 2));
+        origin = Kn == 6 && off == 0u;
+        return (unsigned)Kn * (unsigned)a.P + off;
+    }
+};
+
+// acc += A dd for the block of one neighbour (both vertices)
+__device__ __forceinline__ void pair_madd(const float2 A[9], const float2 dd[3], float2 acc[3]) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        acc[r] = __ffma2_rn(A[3 * r], dd[0], __ffma2_rn(A[3 * r + 1], dd[1], __ffma2_rn(A[3 * r + 2], dd[2], acc[r])));
+}
+
+// acc[3c+r] (cases cb .. cb+C-1) += the part of (K u)_v, in difference form
+// sum_d A_d (u_{v+d} - u_v), of the eight neighbour rows other than the pair's own,
+// u at the pinned origin counted as 0.  Equal to sum_d A_d u_{v+d} in exact arithmetic
+// (the blocks of a row sum to zero), and exact for rigid translations in FP32 too, so
+// the FP32 operator agrees with the FP64 difference-form residual of the refined mode
+// on the near-null translation mode of the pinned problem.  nuv: -u of the pair.
+// r0 .. r1-1: the rows, (dy, dz) with dy fastest.
+template <int C>
+__device__ __forceinline__ void pair_rows(const FineArgs &a, const KeMat &ke, const PairGeo &g, int cb,
+                                          const float2 nuv[3 * C], float2 acc[3 * C], int r0, int r1) {
+#pragma unroll
+    for (int r = r0; r < r1; ++r) {
+        const int dy = r % 3 - 1, dz = r / 3 - 1;
+        bool origin;
+        const unsigned ro = g.row(a, dy, dz, origin);
+        const unsigned ev = ro + (unsigned)a.P;
+        const float *u = a.u + 3 * cb * FVB;
+        const float *po = u + fpos(ro + (unsigned)g.i), *pe = u + fpos(ev + (unsigned)g.i);
+        const float *pm = u + fpos(ro + (unsigned)g.im), *pp = u + fpos(ev + (unsigned)g.ip);
+        if (origin && g.i == 0) pe = zero_planes;
+        if (origin && g.ip == 0) pp = zero_planes;
+        float e0[3 * C], o0[3 * C];
+        float2 A[9];
+        g.block(ke, 3 * r, A);  // dx = -1: the odd vertex's left neighbour is e0
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
             float2 dd[3];
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
-                const float2 un = pinned ? make_float2(0.f, 0.f)
-                                         : make_float2(__ldg(up + (6 * j + m) * FVB), __ldg(up + (6 * j + 3 + m) * FVB));
-                dd[m] = __fadd2_rn(un, nuv2[3 * j + m]);
+                const int q = 3 * c + m;
+                e0[q] = __ldg(pe + q * FVB);
+                dd[m] = make_float2(__fadd_rn(e0[q], nuv[q].x), __fadd_rn(__ldg(pm + q * FVB), nuv[q].y));
             }
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-                acc2[3 * j + r] = __ffma2_rn(make_float2(A[3 * r], A[3 * r]), dd[0],
-                                             __ffma2_rn(make_float2(A[3 * r + 1], A[3 * r + 1]), dd[1],
-                                                        __ffma2_rn(make_float2(A[3 * r + 2], A[3 * r + 2]), dd[2],
-                                                                   acc2[3 * j + r])));
+            pair_madd(A, dd, acc + 3 * c);
         }
-        if (NS) {
-            float dd[3];
+        g.block(ke, 3 * r + 1, A);
 #pragma unroll
-            for (int m = 0; m < 3; ++m) dd[m] = __fadd_rn(pinned ? 0.f : __ldg(up + (6 * NP + m) * FVB), nuv1[m]);
+        for (int c = 0; c < C; ++c) {
+            float2 dd[3];
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
-                acc1[r] = __fmaf_rn(A[3 * r], dd[0], __fmaf_rn(A[3 * r + 1], dd[1], __fmaf_rn(A[3 * r + 2], dd[2], acc1[r])));
+            for (int m = 0; m < 3; ++m) {
+                const int q = 3 * c + m;
+                o0[q] = __ldg(po + q * FVB);
+                dd[m] = make_float2(__fadd_rn(o0[q], nuv[q].x), __fadd_rn(e0[q], nuv[q].y));
+            }
+            pair_madd(A, dd, acc + 3 * c);
+        }
+        g.block(ke, 3 * r + 2, A);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            float2 dd[3];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const int q = 3 * c + m;
+                const float e1 = __ldg(pp + q * FVB);
+                dd[m] = make_float2(__fadd_rn(e1, nuv[q].x), __fadd_rn(o0[q], nuv[q].y));
+            }
+            pair_madd(A, dd, acc + 3 * c);
         }
     }
-#pragma unroll
-    for (int j = 0; j < NP; ++j)
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            acc[6 * j + m] = acc2[3 * j + m].x;
-            acc[6 * j + 3 + m] = acc2[3 * j + m].y;
-        }
-#pragma unroll
-    for (int m = 0; m < 3 * NS; ++m) acc[6 * NP + m] = acc1[m];
 }
 
-// thread -> (vertex p in the colour plane, first case cb) for C cases per thread;
-// the NCASE / C case groups of a vertex block are adjacent CTAs
-// vertex block are adjacent CTAs
-template <int C>
-__device__ __forceinline__ void thread_task(long long &p, int &cb, unsigned bid) {
+// thread -> pair: row block rb of the CTA, row slot and pair index; false for threads
+// without one
+__device__ __forceinline__ bool pair_task(const FineArgs &a, unsigned rb, int &slot, int &i, unsigned &row, int &j,
+                                          int &l) {
+    slot = (int)a.dh0.div(threadIdx.x);
+    i = (int)threadIdx.x - slot * a.h[0];
+    row = rb * (unsigned)a.rows + (unsigned)slot;
+    l = (int)a.dh1.div(row);
+    j = (int)row - l * a.h[1];
+    return slot < a.rows && row < (unsigned)(a.h[1] * a.h[2]);
+}
+
+// the reference's component-wise block Gauss-Seidel step (x, then y, then z,
+// each with the relaxed values of the earlier components) written as an
+// update of u by the residual r = f - K u; rk: w over the diagonal of ks
+__device__ __forceinline__ void gs_step(const float ks[9], const float rk[3], float r0, float r1, float r2, float &u0,
+                                        float &u1, float &u2) {
+    const float d0 = r0 * rk[0];
+    const float d1 = (r1 - ks[3] * d0) * rk[1];
+    const float d2 = (r2 - ks[6] * d0 - ks[7] * d1) * rk[2];
+    u0 += d0;
+    u1 += d1;
+    u2 += d2;
+}
+
+// Two colours of the sweep: the rows of parity K0, their odd vertices (colour K0)
+// first, then, after a barrier, the even ones (colour K0 + 1), whose neighbours in the
+// own row are the new odd values (handed over in shared memory).  Rows of the same
+// parity are never neighbours, so the launch is the two colours' exact Gauss-Seidel
+// order.  The neighbour rows' part of both vertices is formed together.  One launch per
+// colour streamed all of u eight times a sweep (12 GB of DRAM traffic at 256^3) and
+// fetched 17 row halves per 128 vertices from L2; this reads u four times and 18 row
+// halves per 256 vertices.  Bound by load latency and issue (54-58 % of issue slots,
+// 15 warps per SM, DRAM 29 % at 128^3).  Sweep at 256^3 / 128^3 / 64^3: 2.82 / 0.42 / 0.082
+// ms with one colour per launch, 2.29 / 0.33 / 0.060 ms now.
+// bid: the CTA's index in the design's launch; sm: 3 C x TM floats
+template <int K0, int C, int TM>
+__device__ __forceinline__ void fine_gs_block(const FineArgs &a, const KeMat &ke, unsigned bid) {
+    __shared__ float sm[3 * C][TM];
     constexpr int NG = NCASE / C;
-    cb = (int)(bid % NG) * C;
-    p = (long long)(bid / NG) * blockDim.x + threadIdx.x;
-}
-
-// one vertex of the colour sweep; RES (the last colour of a sweep) also writes
-// the residual of the updated vertex, whose neighbours (all of other colours) are
-// final: with acc = sum_d A_d (u_{v+d} - u_v) taken before the update and the
-// blocks of a row summing to zero, f - K u after u_v += e is (f - acc) - A_0 e,
-// e the change actually stored.  nrm[c] gathers the weighted squared residual.
-template <int K, int C, bool RES>
-__device__ __forceinline__ void fine_gs_vertex(const FineArgs &a, const KeMat &ke, long long p, int cb,
-                                               double nrm[C]) {
-    const long long me = (long long)K * a.P + p;
-    if (K == 7 && p == 0) {  // the pinned origin (grid.cu:445-447, 545)
+    const int cb = (int)(bid % NG) * C;
+    int slot, i, j, l;
+    unsigned row;
+    const bool on = pair_task(a, bid / NG, slot, i, row, j, l);
+    if (bid % NG == 0 && threadIdx.x < 10) {  // u of all colours, f of the two swept
+        const unsigned r0 = (bid / NG + GS_AHEAD) * (unsigned)a.rows, rows = (unsigned)(a.h[1] * a.h[2]);
+        if (r0 < rows) {
+            const unsigned r1 = min(rows, r0 + (unsigned)a.rows), t = threadIdx.x, k = t < 8 ? t : K0 + t - 8;
+            const unsigned long long v0 = (unsigned long long)k * a.P + r0 * (unsigned)a.h[0];
+            prefetch_field(t < 8 ? a.u : a.f, v0, v0 + (r1 - r0) * (unsigned)a.h[0]);
+        }
+    }
+    const unsigned vo = (unsigned)K0 * (unsigned)a.P + row * (unsigned)a.h[0] + (unsigned)i;
+    const size_t po = fpos(vo) + 3 * cb * FVB, pe = fpos(vo + (unsigned)a.P) + 3 * cb * FVB;
+    float *uo = a.u + po, *ue = a.u + pe;
+    const float *fo = a.f + po, *fe = a.f + pe;
+    float2 nuv[3 * C], acc[3 * C], A[9];
+    const PairGeo g(a, K0, on ? i : 0, on ? j : 0, on ? l : 0);
+    bool origin;
+    const unsigned ro = g.row(a, 0, 0, origin);
+    if (on) {
 #pragma unroll
         for (int q = 0; q < 3 * C; ++q) {
-            a.u[fidx(3 * cb + q, me)] = 0.f;
-            if (RES) a.r[fidx(3 * cb + q, me)] = 0.f;
+            // the pinned origin counts as 0
+            nuv[q] = make_float2(-uo[q * FVB], origin && i == 0 ? -0.f : -ue[q * FVB]);
+            acc[q] = make_float2(0.f, 0.f);
         }
-        return;
-    }
-    const VertexGeo<K> g(a, p);
-    float uv[3 * C];
+        pair_rows<C>(a, ke, g, cb, nuv, acc, 0, 4);
+        pair_rows<C>(a, ke, g, cb, nuv, acc, 5, 9);
+        // own row, odd vertex: the even neighbours' old values
+        {
+            const float *pp = a.u + fidx(3 * cb, ro + (unsigned)a.P + (unsigned)g.ip);
+            float2 B[9];
+            g.block(ke, 12, A);
+            g.block(ke, 14, B);
+            const bool z1 = origin && g.ip == 0;
 #pragma unroll
-    for (int q = 0; q < 3 * C; ++q) uv[q] = a.u[fidx(3 * cb + q, me)];
-    float acc[3 * C];
-    fine_apply<K, C>(a, ke, g, cb, uv, acc);
-    float ks[9];
-    g.block(ke, 13, ks);
-    const float w = a.w;
-    double mult = 0;
-    if (RES) {
-        constexpr int px = (K & 1) ^ 1, py = ((K >> 1) & 1) ^ 1, pz = ((K >> 2) & 1) ^ 1;
-        int i, j, l;
-        plane_coords(a, p, i, j, l);
-        mult = (double)(axis_mult(2 * i + px, a.n[0]) * axis_mult(2 * j + py, a.n[1]) * axis_mult(2 * l + pz, a.n[2]));
+            for (int c = 0; c < C; ++c) {
+                float dl[3], dr[3];
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    const int q = 3 * c + m;
+                    dl[m] = nuv[q].x - nuv[q].y;
+                    dr[m] = (z1 ? 0.f : pp[q * FVB]) + nuv[q].x;
+                }
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    float v = acc[3 * c + r].x;
+                    v = fmaf(A[3 * r].x, dl[0], fmaf(A[3 * r + 1].x, dl[1], fmaf(A[3 * r + 2].x, dl[2], v)));
+                    acc[3 * c + r].x = fmaf(B[3 * r].x, dr[0], fmaf(B[3 * r + 1].x, dr[1], fmaf(B[3 * r + 2].x, dr[2], v)));
+                }
+            }
+        }
+        g.block(ke, 13, A);
+        float ks[9], rk[3];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) ks[e] = A[e].x;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) rk[m] = a.w / ks[4 * m];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            float u0 = -nuv[3 * c].x, u1 = -nuv[3 * c + 1].x, u2 = -nuv[3 * c + 2].x;
+            gs_step(ks, rk, fo[3 * c * FVB] - acc[3 * c].x, fo[(3 * c + 1) * FVB] - acc[3 * c + 1].x,
+                    fo[(3 * c + 2) * FVB] - acc[3 * c + 2].x, u0, u1, u2);
+            sm[3 * c][threadIdx.x] = u0;
+            sm[3 * c + 1][threadIdx.x] = u1;
+            sm[3 * c + 2][threadIdx.x] = u2;
+        }
     }
-    // the reference's component-wise block Gauss-Seidel step (x, then y, then z,
-    // each with the relaxed values of the earlier components) written as an
-    // update of u by the residual r = f - K u
+    __syncthreads();
+    if (!on) return;
+    const int tm = (int)threadIdx.x - i + g.im;
+    float2 B[9];
+    g.block(ke, 14, B);
+    float ks[9], rk[3];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) ks[e] = A[e].y;
+    g.block(ke, 12, A);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) rk[m] = a.w / ks[4 * m];
+    const bool pinned = origin && i == 0;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-        const long long o = fidx(3 * (cb + c), me);
-        const float r0 = a.f[o] - acc[3 * c], r1 = a.f[o + FVB] - acc[3 * c + 1], r2 = a.f[o + 2 * FVB] - acc[3 * c + 2];
-        const float d0 = w * r0 / ks[0];
-        const float d1 = w * (r1 - ks[3] * d0) / ks[4];
-        const float d2 = w * (r2 - ks[6] * d0 - ks[7] * d1) / ks[8];
-        const float n0 = uv[3 * c] + d0, n1 = uv[3 * c + 1] + d1, n2 = uv[3 * c + 2] + d2;
-        a.u[o] = n0;
-        a.u[o + FVB] = n1;
-        a.u[o + 2 * FVB] = n2;
-        if (RES) {
-            const float e0 = n0 - uv[3 * c], e1 = n1 - uv[3 * c + 1], e2 = n2 - uv[3 * c + 2];
-            const float q0 = r0 - fmaf(ks[2], e2, fmaf(ks[1], e1, ks[0] * e0));
-            const float q1 = r1 - fmaf(ks[5], e2, fmaf(ks[4], e1, ks[3] * e0));
-            const float q2 = r2 - fmaf(ks[8], e2, fmaf(ks[7], e1, ks[6] * e0));
-            a.r[o] = q0;
-            a.r[o + FVB] = q1;
-            a.r[o + 2 * FVB] = q2;
-            nrm[c] += mult * ((double)q0 * q0 + (double)q1 * q1 + (double)q2 * q2);
+        float dl[3], dr[3], v[3];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const float un = sm[3 * c + m][threadIdx.x];
+            uo[(3 * c + m) * FVB] = un;
+            dl[m] = sm[3 * c + m][tm] + nuv[3 * c + m].y;
+            dr[m] = un + nuv[3 * c + m].y;
         }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            v[r] = acc[3 * c + r].y;
+            v[r] = fmaf(A[3 * r].y, dl[0], fmaf(A[3 * r + 1].y, dl[1], fmaf(A[3 * r + 2].y, dl[2], v[r])));
+            v[r] = fmaf(B[3 * r].y, dr[0], fmaf(B[3 * r + 1].y, dr[1], fmaf(B[3 * r + 2].y, dr[2], v[r])));
+        }
+        float u0 = -nuv[3 * c].y, u1 = -nuv[3 * c + 1].y, u2 = -nuv[3 * c + 2].y;
+        gs_step(ks, rk, fe[3 * c * FVB] - v[0], fe[(3 * c + 1) * FVB] - v[1], fe[(3 * c + 2) * FVB] - v[2], u0, u1, u2);
+        // the pinned origin stays zero (grid.cu:445-447, 545)
+        ue[3 * c * FVB] = pinned ? 0.f : u0;
+        ue[(3 * c + 1) * FVB] = pinned ? 0.f : u1;
+        ue[(3 * c + 2) * FVB] = pinned ? 0.f : u2;
     }
 }
 
-// RES: the per-CTA norm partials go to the rows the residual of colour 7 would
-// write (row 7 * (CTAs per colour of the residual) + CTA of the colour, one row
-// per group of CPT cases, zeros for the other cases).  bid / nblk: the CTA's index
-// and the CTA count of the design's launch (blockIdx.x / gridDim.x, or the slice
-// of a batched launch, k_fine_gs_batch)
-template <int K, int C, bool RES>
-__device__ __forceinline__ void fine_gs_block(const FineArgs &a, const KeMat &ke, double *partial, unsigned bid,
-                                              unsigned nblk) {
-    long long p;
-    int cb;
-    thread_task<C>(p, cb, bid);
+// TM: threads per CTA at most; MB: CTAs per SM
+template <int K0, int C, int TM, int MB>
+__global__ void __launch_bounds__(TM, MB) k_fine_gs(FineArgs a, const __grid_constant__ KeMat ke) {
+    fine_gs_block<K0, C, TM>(a, ke, blockIdx.x);
+}
+
+// Residual of all rows in one launch (there is no order between colours), the row
+// parity the block index modulo 4 and a run-time value of one code body: the CTAs of
+// neighbouring rows run together and read each other's rows while they are in L2.
+// 256^3: 3.48 ms with one vertex per thread (2.95 ms without the last colour, which the
+// sweep then wrote), 2.47 ms now; three cases per thread or other register budgets
+// measured 2.73 to 3.26.
+// norm partials: the six weighted squared norms of every row of vertices, row
+// K0/2 * (rows of a parity) + row, summed in an order that depends on the row length
+// alone (the same in any launch shape and in lockstep batches).
+template <int C, int TM>
+__device__ __forceinline__ void fine_residual_block(const FineArgs &a, const KeMat &ke, double *partial, unsigned bid) {
+    constexpr int NG = NCASE / C;
+    const int K0 = (int)(bid & 3u) * 2;
+    const unsigned bx = bid >> 2;
+    const int cb = (int)(bx % NG) * C;
+    int slot, i, j, l;
+    unsigned row;
+    const bool on = pair_task(a, bx / NG, slot, i, row, j, l);
+    if (bx % NG == 0 && threadIdx.x < 4) {  // u and f of the row parity's two colours
+        const unsigned r0 = (bx / NG + RES_AHEAD) * (unsigned)a.rows, rows = (unsigned)(a.h[1] * a.h[2]);
+        if (r0 < rows) {
+            const unsigned r1 = min(rows, r0 + (unsigned)a.rows), t = threadIdx.x, k = (unsigned)K0 + (t & 1);
+            const unsigned long long v0 = (unsigned long long)k * a.P + r0 * (unsigned)a.h[0];
+            prefetch_field(t < 2 ? a.u : a.f, v0, v0 + (r1 - r0) * (unsigned)a.h[0]);
+        }
+    }
     double nrm[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) nrm[c] = 0;
-    if (!RES) {
-        if (p < a.P) fine_gs_vertex<K, C, false>(a, ke, p, cb, nrm);
-        return;
-    }
-    static_assert(!RES || (K == 7 && C % CPT == 0), "the fused residual is the last colour's");
-    if (p < a.P) fine_gs_vertex<K, C, RES>(a, ke, p, cb, nrm);
-    __shared__ double sm[C][FBS / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (on) {
+        const unsigned vo = (unsigned)K0 * (unsigned)a.P + row * (unsigned)a.h[0] + (unsigned)i;
+        const size_t oo = fpos(vo) + 3 * cb * FVB, oe = fpos(vo + (unsigned)a.P) + 3 * cb * FVB;
+        const float *uo = a.u + oo, *ue = a.u + oe;
+        const PairGeo g(a, K0, i, j, l);
+        bool origin;
+        const unsigned ro = g.row(a, 0, 0, origin);
+        const bool pinned = origin && i == 0;
+        float2 nuv[3 * C], acc[3 * C];
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-        const double v = warp_sum(nrm[c]);
-        if (lane == 0) sm[c][wid] = v;
-    }
-    __syncthreads();
-    constexpr int NG = NCASE / C, NGR = NCASE / CPT;  // case groups of this launch / of the residual
-    const long long pb = bid / NG, npb = nblk / NG;  // vertex block, vertex blocks
-    if (threadIdx.x < (C / CPT) * NCASE) {
-        const int gl = threadIdx.x / NCASE, q = threadIdx.x % NCASE;
-        const int g = cb / CPT + gl;  // the residual's case group of this row
-        double v = 0;
-        if (q >= g * CPT && q < (g + 1) * CPT)
-#pragma unroll
-            for (int w = 0; w < FBS / 32; ++w) v += sm[q - cb][w];
-        partial[((7 * npb + pb) * NGR + g) * NCASE + q] = v;
-    }
-}
-
-template <int K, int C, int MINB, bool RES>
-__global__ void __launch_bounds__(FBS, MINB) k_fine_gs(FineArgs a, const __grid_constant__ KeMat ke,
-                                                    double *partial) {
-    fine_gs_block<K, C, RES>(a, ke, partial, blockIdx.x, gridDim.x);
-}
-
-template <int KC>
-__device__ __forceinline__ void fine_residual_vertex(const FineArgs &a, const KeMat &ke, long long p, int cb,
-                                                     double nrm[CPT], int kr = KC) {
-    const int K = KC >= 0 ? KC : kr;
-    const long long me = (long long)K * a.P + p;
-    if (K == 7 && p == 0) {
-#pragma unroll
-        for (int q = 0; q < 3 * CPT; ++q) a.r[fidx(3 * cb + q, me)] = 0.f;
-        return;
-    }
-    const VertexGeo<KC> g(a, p, K);
-    float uv[3 * CPT];
-#pragma unroll
-    for (int q = 0; q < 3 * CPT; ++q) uv[q] = __ldg(a.u + fidx(3 * cb + q, me));
-    float acc[3 * CPT];
-    fine_apply<KC, CPT>(a, ke, g, cb, uv, acc);
-    const int px = (K & 1) ^ 1, py = ((K >> 1) & 1) ^ 1, pz = ((K >> 2) & 1) ^ 1;
-    int i, j, l;
-    plane_coords(a, p, i, j, l);
-    const double mult = (double)(axis_mult(2 * i + px, a.n[0]) * axis_mult(2 * j + py, a.n[1]) *
-                                 axis_mult(2 * l + pz, a.n[2]));
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-        double s2 = 0;
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            const long long o = fidx(3 * (cb + c) + m, me);
-            const float rv = a.f[o] - acc[3 * c + m];
-            a.r[o] = rv;
-            s2 += (double)rv * rv;
+        for (int q = 0; q < 3 * C; ++q) {
+            nuv[q] = make_float2(-__ldg(uo + q * FVB), pinned ? -0.f : -__ldg(ue + q * FVB));
+            acc[q] = make_float2(0.f, 0.f);
         }
-        nrm[c] += mult * s2;
+        pair_rows<C>(a, ke, g, cb, nuv, acc, 0, 4);
+        {
+            const float *pm = a.u + fidx(3 * cb, ro + (unsigned)g.im);
+            const float *pp = a.u + fidx(3 * cb, ro + (unsigned)a.P + (unsigned)g.ip);
+            const bool z1 = origin && g.ip == 0;
+            float2 A[9], B[9];
+            g.block(ke, 12, A);
+            g.block(ke, 14, B);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                float2 dl[3], dr[3];
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    const int q = 3 * c + m;
+                    dl[m] = make_float2(nuv[q].x - nuv[q].y, __ldg(pm + q * FVB) + nuv[q].y);
+                    dr[m] = make_float2((z1 ? 0.f : __ldg(pp + q * FVB)) + nuv[q].x, nuv[q].y - nuv[q].x);
+                }
+                pair_madd(A, dl, acc + 3 * c);
+                pair_madd(B, dr, acc + 3 * c);
+            }
+        }
+        pair_rows<C>(a, ke, g, cb, nuv, acc, 5, 9);
+        const int my = axis_mult(2 * j + (((K0 >> 1) & 1) ^ 1), a.n[1]) * axis_mult(2 * l + (((K0 >> 2) & 1) ^ 1), a.n[2]);
+        const double mo = (double)(my * axis_mult(2 * i + 1, a.n[0])), me = (double)(my * axis_mult(2 * i, a.n[0]));
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            double so = 0, se = 0;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const int q = 3 * c + m;
+                const float ro_ = a.f[oo + q * FVB] - acc[q].x;
+                const float re_ = pinned ? 0.f : a.f[oe + q * FVB] - acc[q].y;
+                a.r[oo + q * FVB] = ro_;
+                a.r[oe + q * FVB] = re_;
+                so += (double)ro_ * ro_;
+                se += (double)re_ * re_;
+            }
+            nrm[c] = mo * so + me * se;
+        }
+    }
+    if (!partial) return;
+    __shared__ double sm[C][TM];
+#pragma unroll
+    for (int c = 0; c < C; ++c) sm[c][threadIdx.x] = nrm[c];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const unsigned rows = (unsigned)(a.h[1] * a.h[2]), first = bx / NG * (unsigned)a.rows;
+    for (int t = threadIdx.x >> 5; t < a.rows * C; t += nw) {
+        const int rr = t / C, c = t % C;
+        if (first + (unsigned)rr >= rows) continue;
+        double v = 0;
+        for (int e = lane; e < a.h[0]; e += 32) v += sm[c][rr * a.h[0] + e];
+        v = warp_sum(v);
+        if (lane == 0) partial[((long long)(K0 / 2) * rows + first + rr) * NCASE + cb + c] = v;
     }
 }
 
-// The residual has no order between the colours, so all eight run in one launch
-// with the colour the block index modulo the colour count (8, or 7 when the sweep
-// before it wrote colour 7's residual): the eight CTAs of one
-// vertex block cover a 2x2x2 neighbourhood of the grid and read each other's rows
-// while they are in L2, where one launch per colour would stream the whole u
-// field from HBM once per colour.  The colour is a run-time value of one code
-// body (VertexGeo<-1>): eight compile-time colour bodies resident on an SM at
-// once thrash the instruction cache (2.5x slower at 256^3), while the run-time
-// colour costs a few integer operations per neighbour.  One thread per vertex
-// (six cases) is slower here too: 3.55 against 3.11 ms per 256^3 residual.  The
-// per-CTA norm partials of the CTA's two cases go to row colour * (CTAs per
-// colour) + CTA of the colour, zeros for the other cases, as with one launch per
-// colour, so the norms are summed in the same order.
+template <int C, int TM, int MB>
+__global__ void __launch_bounds__(TM, MB) k_fine_residual(FineArgs a, const __grid_constant__ KeMat ke,
+                                                          double *partial) {
+    fine_residual_block<C, TM>(a, ke, partial, blockIdx.x);
+}
+
+// thread -> (colour, vertex p of its plane, first case) of the FP64-solution residual:
+// the colour the block index modulo 8, so the CTAs of one vertex block read each
+// other's rows while they are in L2
 template <int C>
-__device__ __forceinline__ void colour_task(long long &p, int &cb, int &K, unsigned &bx, unsigned bid,
-                                            unsigned ncol = 8) {
+__device__ __forceinline__ void colour_task(long long &p, int &cb, int &K, unsigned bid) {
     constexpr int NG = NCASE / C;
-    K = (int)(bid % ncol);
-    bx = bid / ncol;
+    K = (int)(bid % 8);
+    const unsigned bx = bid / 8;
     cb = (int)(bx % NG) * C;
     p = (long long)(bx / NG) * blockDim.x + threadIdx.x;
-}
-
-template <unsigned NCOL>  // colours 0 .. NCOL-1 (8, or 7 after a sweep that did colour 7's)
-__device__ __forceinline__ void fine_residual_block(const FineArgs &a, const KeMat &ke, double *partial, unsigned bid,
-                                                    unsigned nblk) {
-    constexpr unsigned ncol = NCOL;
-    long long p;
-    int cb, K;
-    unsigned bx;
-    colour_task<CPT>(p, cb, K, bx, bid, ncol);
-    double nrm[CPT] = {};
-    if (p < a.P) fine_residual_vertex<-1>(a, ke, p, cb, nrm, K);
-    if (!partial) return;
-    __shared__ double sm[CPT][FBS / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-        const double v = warp_sum(nrm[c]);
-        if (lane == 0) sm[c][wid] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < NCASE) {
-        const int q = threadIdx.x;
-        double v = 0;
-        if (q >= cb && q < cb + CPT)
-#pragma unroll
-            for (int w = 0; w < FBS / 32; ++w) v += sm[q - cb][w];
-        partial[((long long)K * (nblk / ncol) + bx) * NCASE + q] = v;
-    }
-}
-
-template <unsigned NCOL>
-__global__ void __launch_bounds__(FBS, RES_MINB) k_fine_residual(FineArgs a, const __grid_constant__ KeMat ke,
-                                                       double *partial) {
-    fine_residual_block<NCOL>(a, ke, partial, blockIdx.x, gridDim.x);
 }
 
 // ---- refined precision: residual of an FP64 solution ----------------------------
@@ -549,8 +719,7 @@ __global__ void __launch_bounds__(FBS, MB) k_fine_residual64(FineArgs a, const _
                                                          const double *__restrict__ u64) {
     long long p;
     int cb, K;
-    unsigned bx;
-    colour_task<C64>(p, cb, K, bx, blockIdx.x);  // all colours in one launch, colour-minor
+    colour_task<C64>(p, cb, K, blockIdx.x);  // all colours in one launch, colour-minor
     if (p >= a.P) return;
     fine_residual64_vertex<-1, EXACT, C64>(a, ke, ke64, u64, p, cb, K);
 }
@@ -594,79 +763,61 @@ static FineArgs make_args(const Level &L, const float *rho) {
     a.w = 1.f;
     a.dh0 = FastDiv((unsigned)a.h[0]);
     a.dh1 = FastDiv((unsigned)a.h[1]);
+    a.rows = pair_shape(a.h[0]).rows;
     return a;
 }
 
 static unsigned task_blocks(const FineArgs &a, int cpt) { return (unsigned)(((a.P + FBS - 1) / FBS) * (NCASE / cpt)); }
 
-int fine_residual_blocks(const Level &L) { return (int)(((L.P.nv / 8 + FBS - 1) / FBS) * (NCASE / CPT) * 8); }
+// row blocks of a launch over the rows of one parity, for CTAs of a.rows rows
+static unsigned pair_blocks(const FineArgs &a) { return (unsigned)((a.h[1] * a.h[2] + a.rows - 1) / a.rows); }
 
-// the colour sweep in launch shape v: 0 = one thread per vertex with all six
-// cases (4 CTAs/SM), 1 = three threads per vertex with two cases each (5 CTAs/SM),
-// 2 = three cases per thread (two threads per vertex, one case pair and one scalar
-// case) at 5 CTAs/SM, 3 = two cases per thread at 6 CTAs/SM (fewer registers);
-// all give the same result to the last bit
-template <int C, int MINB>
-static void fine_gs_sweep(const FineArgs &a, const KeMat &ke, cudaStream_t s) {
-    const unsigned nb = task_blocks(a, C);
-    k_fine_gs<0, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<1, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<2, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<3, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<4, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<5, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<6, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<7, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
+int fine_residual_blocks(const Level &L) { return L.P.n[1] * L.P.n[2]; }
+
+// The colour sweep in launch shape v: load cases per thread and CTAs of 128 threads
+// per SM; all give the same result to the last bit (256^3 / 64^3: shape 0 2.29 / 0.060,
+// 1 2.50 / 0.058, 2 2.61 / 0.066, 3 2.57 / 0.065 ms)
+template <int C, int TM, int MB>
+static void fine_gs_sweep(const FineArgs &a, const KeMat &ke, unsigned nt, cudaStream_t s) {
+    const unsigned nb = pair_blocks(a) * (NCASE / C);
+    k_fine_gs<0, C, TM, MB><<<nb, nt, 0, s>>>(a, ke);
+    k_fine_gs<2, C, TM, MB><<<nb, nt, 0, s>>>(a, ke);
+    k_fine_gs<4, C, TM, MB><<<nb, nt, 0, s>>>(a, ke);
+    k_fine_gs<6, C, TM, MB><<<nb, nt, 0, s>>>(a, ke);
+}
+
+// CTAs of up to 128, 256 or 512 threads (pair_shape), with the same threads per SM
+template <int C, int MB>
+static void fine_gs_shape(const FineArgs &a, const KeMat &ke, cudaStream_t s) {
+    const unsigned nt = (unsigned)pair_shape(a.h[0]).threads;
+    if (nt <= 128) fine_gs_sweep<C, 128, MB>(a, ke, nt, s);
+    else if (nt <= 256) fine_gs_sweep<C, 256, MB / 2>(a, ke, nt, s);
+    else fine_gs_sweep<C, 512, 1>(a, ke, nt, s);
 }
 
 void launch_fine_gs(const Level &L, const float *rho, const KeMat &ke, float w, cudaStream_t s) {
     FineArgs a = make_args(L, rho);
     a.w = w;
     switch (L.gs_shape) {
-    case 1: fine_gs_sweep<2, 5>(a, ke, s); break;
-    case 2: fine_gs_sweep<3, 5>(a, ke, s); break;
-    case 3: fine_gs_sweep<2, 6>(a, ke, s); break;
-    default: fine_gs_sweep<6, 4>(a, ke, s); break;
+    case 1: fine_gs_shape<6, 2>(a, ke, s); break;
+    case 2: fine_gs_shape<2, 5>(a, ke, s); break;
+    case 3: fine_gs_shape<3, 3>(a, ke, s); break;
+    default: fine_gs_shape<3, 4>(a, ke, s); break;
     }
-}
-
-// a sweep followed by the residual (the down leg of a V-cycle): the last colour's
-// launch writes its own residual and norm partials, the residual launch covers
-// the other seven colours
-template <int C, int MINB>
-static void fine_gs_sweep_res(const FineArgs &a, const KeMat &ke, double *partial, cudaStream_t s) {
-    const unsigned nb = task_blocks(a, C);
-    k_fine_gs<0, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<1, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<2, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<3, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<4, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<5, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    k_fine_gs<6, C, MINB, false><<<nb, FBS, 0, s>>>(a, ke, nullptr);
-    // the last colour writes its residual with the norm partials of the residual's
-    // case pairs: an odd case count per thread takes the six-case kernel for it
-    constexpr int CR = (C % CPT == 0) ? C : 6, MR = (C % CPT == 0) ? MINB : 4;
-    k_fine_gs<7, CR, MR, true><<<task_blocks(a, CR), FBS, 0, s>>>(a, ke, partial);
-    k_fine_residual<7><<<task_blocks(a, CPT) * 7, FBS, 0, s>>>(a, ke, partial);
 }
 
 void launch_fine_gs_residual(const Level &L, const float *rho, const KeMat &ke, float w, double *norm_partial,
                              cudaStream_t s) {
-    FineArgs a = make_args(L, rho);
-    a.w = w;
-    switch (L.gs_shape) {
-    case 1: fine_gs_sweep_res<2, 5>(a, ke, norm_partial, s); break;
-    case 2: fine_gs_sweep_res<3, 5>(a, ke, norm_partial, s); break;
-    case 3: fine_gs_sweep_res<2, 6>(a, ke, norm_partial, s); break;
-    default: fine_gs_sweep_res<6, 4>(a, ke, norm_partial, s); break;
-    }
+    launch_fine_gs(L, rho, ke, w, s);
+    launch_fine_residual(L, rho, ke, norm_partial, s);
 }
 
-void launch_fine_residual(const Level &L, const float *rho, const KeMat &ke, double *norm_partial, int nblk_norm,
-                          cudaStream_t s) {
-    FineArgs a = make_args(L, rho);
-    (void)nblk_norm;
-    k_fine_residual<8><<<task_blocks(a, CPT) * 8, FBS, 0, s>>>(a, ke, norm_partial);
+void launch_fine_residual(const Level &L, const float *rho, const KeMat &ke, double *norm_partial, cudaStream_t s) {
+    const FineArgs a = make_args(L, rho);
+    const unsigned nb = pair_blocks(a) * (NCASE / CPT) * 4, nt = (unsigned)pair_shape(a.h[0]).threads;
+    if (nt <= 128) k_fine_residual<CPT, 128, RES_MINB><<<nb, nt, 0, s>>>(a, ke, norm_partial);
+    else if (nt <= 256) k_fine_residual<CPT, 256, RES_MINB / 2><<<nb, nt, 0, s>>>(a, ke, norm_partial);
+    else k_fine_residual<CPT, 512, 1><<<nb, nt, 0, s>>>(a, ke, norm_partial);
 }
 
 void launch_fine_residual64(const Level &L, const float *rho, const KeMat &ke, const KeMat64 &ke64, const float *f,
@@ -883,8 +1034,8 @@ void launch_convert_field(long long nv, const double *src, float *dst, cudaStrea
 // per-CTA body as its own launch would, with its CTA index inside the slice, so
 // every design's fields and norm partials are those of its own launches, to the
 // last bit.  A CTA copies its design's arguments to shared memory once; a design
-// whose flag in `active` is 0 (converged) returns at once.  The sweep runs in
-// launch shape 0 (six cases per thread, 4 CTAs/SM).
+// whose flag in `active` is 0 (converged) returns at once.  All designs of a launch
+// share one CTA size, so a design's rows per CTA can differ from its own launch's.
 struct FineEnt {
     FineArgs a;
     double *partial;  // the design's norm partials
@@ -892,40 +1043,36 @@ struct FineEnt {
     int design;       // its index in the active flags
 };
 struct FineBatchTab {
-    BatchSlices gs;   // CTAs of one colour of the sweep, six cases per thread
-    BatchSlices gs3;  // the same with three cases per thread
-    BatchSlices res;  // CTAs of the seven-colour residual
+    BatchSlices gs;   // CTAs of one sweep launch, three cases per thread
+    BatchSlices gs2;  // the same with two cases per thread
+    BatchSlices res;  // CTAs of the residual
     FineEnt e[BATCH_MAX];
 };
 
-// C cases per thread at MB CTAs per SM: launch shape 0 (C = 6, 4 CTAs/SM) or 1
-// (C = 3, 5 CTAs/SM, one case pair and one scalar case per thread); the colour that
-// writes the residual runs with six cases per thread in both
-template <int K, bool RES, int C, int MB>
-__global__ void __launch_bounds__(FBS, MB) k_fine_gs_batch(const FineBatchTab *__restrict__ t,
-                                                         const int *__restrict__ active,
-                                                         const __grid_constant__ KeMat ke) {
-    static_assert(!RES || C == 6, "the residual-writing colour runs six cases per thread");
+// C cases per thread: launch shape 0 (C = 3, 4 CTAs of 128 threads per SM) or 1 (C = 2, 5)
+template <int K0, int C, int TM, int MB>
+__global__ void __launch_bounds__(TM, MB) k_fine_gs_batch(const FineBatchTab *__restrict__ t,
+                                                        const int *__restrict__ active,
+                                                        const __grid_constant__ KeMat ke) {
     __shared__ __align__(16) unsigned buf[(sizeof(FineArgs) + 3) / 4];
-    const BatchSlices &sl = C == 6 ? t->gs : t->gs3;
+    const BatchSlices &sl = C == 3 ? t->gs : t->gs2;
     const int i = batch_slice(sl, blockIdx.x);
     const FineEnt &en = t->e[i];
     if (!__ldg(&active[en.design])) return;
     const FineArgs &a = stage_args(en.a, buf);
-    const unsigned b0 = __ldg(&sl.start[i]), b1 = __ldg(&sl.start[i + 1]);
-    fine_gs_block<K, C, RES>(a, ke, en.partial, blockIdx.x - b0, b1 - b0);
+    fine_gs_block<K0, C, TM>(a, ke, blockIdx.x - __ldg(&sl.start[i]));
 }
 
-__global__ void __launch_bounds__(FBS, RES_MINB) k_fine_residual_batch(const FineBatchTab *__restrict__ t,
-                                                                      const int *__restrict__ active,
-                                                                      const __grid_constant__ KeMat ke) {
+template <int TM, int MB>
+__global__ void __launch_bounds__(TM, MB) k_fine_residual_batch(const FineBatchTab *__restrict__ t,
+                                                              const int *__restrict__ active,
+                                                              const __grid_constant__ KeMat ke) {
     __shared__ __align__(16) unsigned buf[(sizeof(FineArgs) + 3) / 4];
     const int i = batch_slice(t->res, blockIdx.x);
     const FineEnt &en = t->e[i];
     if (!__ldg(&active[en.design])) return;
     const FineArgs &a = stage_args(en.a, buf);
-    const unsigned b0 = __ldg(&t->res.start[i]), b1 = __ldg(&t->res.start[i + 1]);
-    fine_residual_block<7>(a, ke, en.partial, blockIdx.x - b0, b1 - b0);
+    fine_residual_block<CPT, TM>(a, ke, en.partial, blockIdx.x - __ldg(&t->res.start[i]));
 }
 
 // one CTA per design
@@ -943,17 +1090,23 @@ int fine_batch_create(const Level *const *lv0, const float *const *rho, double *
                       double *const *state, const int *design, int n, bool scratch, BatchTab *out) {
     if (n < 1 || n > BATCH_MAX) return -1;
     FineBatchTab *t = new FineBatchTab();
-    t->gs.n = t->gs3.n = t->res.n = n;
-    t->gs.start[0] = t->gs3.start[0] = t->res.start[0] = 0;
+    t->gs.n = t->gs2.n = t->res.n = n;
+    t->gs.start[0] = t->gs2.start[0] = t->res.start[0] = 0;
+    int hmax = 0;
+    for (int i = 0; i < n; i++) hmax = lv0[i]->P.n[0] / 2 > hmax ? lv0[i]->P.n[0] / 2 : hmax;
+    // one CTA size for all: 128 threads, or the longest row's (lockstep rows: h0 < 256)
+    const int nt = hmax <= 128 ? 128 : 256;
     for (int i = 0; i < n; i++) {
         t->e[i].a = make_args(*lv0[i], rho[i]);
+        t->e[i].a.rows = nt / t->e[i].a.h[0];
         if (scratch) t->e[i].a.u = t->e[i].a.r;
         t->e[i].partial = partial[i];
         t->e[i].state = state[i];
         t->e[i].design = design[i];
-        t->gs.start[i + 1] = t->gs.start[i] + task_blocks(t->e[i].a, 6);
-        t->gs3.start[i + 1] = t->gs3.start[i] + task_blocks(t->e[i].a, 3);
-        t->res.start[i + 1] = t->res.start[i] + task_blocks(t->e[i].a, CPT) * 7;
+        const unsigned rb = pair_blocks(t->e[i].a);
+        t->gs.start[i + 1] = t->gs.start[i] + rb * 2;
+        t->gs2.start[i + 1] = t->gs2.start[i] + rb * 3;
+        t->res.start[i + 1] = t->res.start[i] + rb * (NCASE / CPT) * 4;
     }
     void *d = nullptr;
     int rc = cudaMalloc(&d, sizeof(FineBatchTab)) == cudaSuccess ? 0 : -2;
@@ -963,7 +1116,8 @@ int fine_batch_create(const Level *const *lv0, const float *const *rho, double *
         out->n = n;
         out->grid[0] = t->gs.start[n];
         out->grid[1] = t->res.start[n];
-        out->grid[2] = t->gs3.start[n];
+        out->grid[2] = t->gs2.start[n];
+        out->grid[3] = (unsigned)nt;
     } else if (d) {
         cudaFree(d);
     }
@@ -971,29 +1125,27 @@ int fine_batch_create(const Level *const *lv0, const float *const *rho, double *
     return rc;
 }
 
-template <int C, int MB>
+template <int C, int TM, int MB>
 static void fine_sweep_batch(const BatchTab &t, const KeMat &ke, const int *active, bool residual, cudaStream_t s) {
     const FineBatchTab *d = static_cast<const FineBatchTab *>(t.dev);
-    const unsigned g = C == 6 ? t.grid[0] : t.grid[2];
-    k_fine_gs_batch<0, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    k_fine_gs_batch<1, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    k_fine_gs_batch<2, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    k_fine_gs_batch<3, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    k_fine_gs_batch<4, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    k_fine_gs_batch<5, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    k_fine_gs_batch<6, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    if (residual) {
-        k_fine_gs_batch<7, true, 6, 4><<<t.grid[0], FBS, 0, s>>>(d, active, ke);
-        k_fine_residual_batch<<<t.grid[1], FBS, 0, s>>>(d, active, ke);
-    } else {
-        k_fine_gs_batch<7, false, C, MB><<<g, FBS, 0, s>>>(d, active, ke);
-    }
+    const unsigned g = C == 3 ? t.grid[0] : t.grid[2];
+    k_fine_gs_batch<0, C, TM, MB><<<g, TM, 0, s>>>(d, active, ke);
+    k_fine_gs_batch<2, C, TM, MB><<<g, TM, 0, s>>>(d, active, ke);
+    k_fine_gs_batch<4, C, TM, MB><<<g, TM, 0, s>>>(d, active, ke);
+    k_fine_gs_batch<6, C, TM, MB><<<g, TM, 0, s>>>(d, active, ke);
+    constexpr int MR = TM == 128 ? RES_MINB : RES_MINB / 2;
+    if (residual) k_fine_residual_batch<TM, MR><<<t.grid[1], TM, 0, s>>>(d, active, ke);
 }
 
 void launch_fine_sweep_batch(const BatchTab &t, const KeMat &ke, const int *active, bool residual, int shape,
                              cudaStream_t s) {
-    if (shape == 1) fine_sweep_batch<3, 5>(t, ke, active, residual, s);
-    else fine_sweep_batch<6, 4>(t, ke, active, residual, s);
+    if (t.grid[3] == 128) {
+        if (shape == 1) fine_sweep_batch<2, 128, 5>(t, ke, active, residual, s);
+        else fine_sweep_batch<3, 128, 4>(t, ke, active, residual, s);
+    } else {
+        if (shape == 1) fine_sweep_batch<2, 256, 2>(t, ke, active, residual, s);
+        else fine_sweep_batch<3, 256, 2>(t, ke, active, residual, s);
+    }
 }
 
 void launch_pin_deflate_batch(const BatchTab &t, const KeMat &ke, const int *active, cudaStream_t s) {
