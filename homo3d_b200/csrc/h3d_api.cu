@@ -219,6 +219,10 @@ int fail(h3d_handle *h, int code, const std::string &msg) {
 
 int ensure_tmp(h3d_handle *h, size_t nfloat) {
     if (h->tmp_n >= nfloat) return H3D_OK;
+    if (h->dgraph) {  // the design-step graph holds the old buffer's address
+        cudaGraphExecDestroy(h->dgraph);
+        h->dgraph = nullptr;
+    }
     if (h->tmp) cudaFree(h->tmp);
     h->tmp = nullptr;
     h->tmp_n = 0;
@@ -1892,9 +1896,9 @@ int h3d_oc_filter(h3d_handle *h, float *sens_dev, const float *rho_dev, const in
     CK(cudaSetDevice(h->device));
     if (pitchT < 0) pitchT = reso[0];
     const size_t n = (size_t)pitchT * reso[1] * reso[2];
-    if (int e = ensure_tmp(h, n)) return e;
+    if (int e = ensure_tmp(h, n + window_table_floats(radius))) return e;
     CK(cudaMemsetAsync(h->tmp, 0, sizeof(float) * n, h->stream));
-    launch_filter(reso, pitchT, sens_dev, rho_dev, h->tmp, radius, periodic, h->stream);
+    launch_filter(reso, pitchT, sens_dev, rho_dev, h->tmp, radius, periodic, h->tmp + n, h->stream);
     CKL();
     CK(cudaMemcpyAsync(sens_dev, h->tmp, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream));
     return H3D_OK;
@@ -1966,8 +1970,8 @@ int h3d_conv_radial(h3d_handle *h, const float *in_dev, float *out_dev, const in
         return fail(h, H3D_ERR_ARG, "periodic window wider than the grid");
     CK(cudaSetDevice(h->device));
     const size_t ne = (size_t)reso[0] * reso[1] * reso[2];
-    if (int e = ensure_tmp(h, ne)) return e;
-    launch_conv_radial(reso, in_dev, out_dev, h->tmp, radius, periodic, adjoint, h->stream);
+    if (int e = ensure_tmp(h, ne + window_table_floats(radius))) return e;
+    launch_conv_radial(reso, in_dev, out_dev, h->tmp, radius, periodic, adjoint, h->tmp + ne, h->stream);
     CKL();
     return H3D_OK;
 }
@@ -1982,7 +1986,7 @@ int h3d_design_step(h3d_handle *h, const float dC[36], float *rho_dev, float *se
     if (!(prm->volratio > 0 && prm->volratio <= 1)) return fail(h, H3D_ERR_ARG, "volratio outside (0, 1]");
     CK(cudaSetDevice(h->device));
     const long long ne = (long long)n[0] * n[1] * n[2];
-    if (int e = ensure_tmp(h, (size_t)ne)) return e;
+    if (int e = ensure_tmp(h, (size_t)ne + window_table_floats(std::max(prm->filter_radius, 0.f)))) return e;
     if (!h->d_dcw) CK(cudaMalloc(&h->d_dcw, sizeof(float) * 32));
     if (!h->h_dcw) CK(cudaMallocHost(&h->h_dcw, sizeof(float) * 32));
     if (h->dgraph && (h->dkey_rho != rho_dev || h->dkey_sens != sens_dev ||
@@ -2005,7 +2009,7 @@ int h3d_design_step(h3d_handle *h, const float dC[36], float *rho_dev, float *se
         if (prm->sym >= 0) launch_symmetrize(n, sens_dev, prm->sym, s);
         if (prm->filter_radius > 0) {
             cudaMemsetAsync(h->tmp, 0, sizeof(float) * ne, s);
-            launch_filter(n, n[0], sens_dev, rho_dev, h->tmp, prm->filter_radius, prm->filter_periodic, s);
+            launch_filter(n, n[0], sens_dev, rho_dev, h->tmp, prm->filter_radius, prm->filter_periodic, h->tmp + ne, s);
             cudaMemcpyAsync(sens_dev, h->tmp, sizeof(float) * ne, cudaMemcpyDeviceToDevice, s);
         }
         launch_oc(sens_dev, rho_dev, h->tmp, ne, prm->volratio, prm->min_rho, prm->step_limit, prm->damp, h->partial,
