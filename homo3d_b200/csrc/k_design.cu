@@ -45,9 +45,41 @@ void launch_density_in(const int n[3], const float *src, int pitch, float *dst, 
 }
 
 // ---- OC ----------------------------------------------------------------------
-// scratch layout: [0] lo, [1] hi, [2] done, [3] g, [4..] partial sums
+// scratch layout: [0] lo, [1] hi, [2] done, [3] arrival counter, [4..] partial sums.
+// The CTA of a pass that arrives last combines the partials (in a fixed order) and
+// takes the decision, so a bisection step is one launch; a second launch whose one
+// thread added the 1184 partials took 15-18 us a step.
 constexpr int OC_BS = 256;
 constexpr int OC_NB = 1184;  // 8 blocks per SM on 148 SMs
+
+// whether this CTA is the last of its launch to arrive (the others' writes are then
+// visible); every thread must call it, and the counter is left at zero
+__device__ __forceinline__ bool last_cta(double *st) {
+    __shared__ bool last;
+    unsigned *count = reinterpret_cast<unsigned *>(st + 3);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+        if (last) *count = 0u;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// the sum of the launch's partials st[4 ..], in thread 0 of an OC_BS-thread CTA
+__device__ __forceinline__ double sum_partials(const double *st, int nb) {
+    __shared__ double sm[OC_BS / 32];
+    double s = 0;
+    for (int b = threadIdx.x; b < nb; b += OC_BS) s += __ldcg(&st[4 + b]);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < OC_BS / 32; ++w) s += sm[w];
+    return s;
+}
 
 __global__ void __launch_bounds__(OC_BS) k_oc_maxabs(const float *__restrict__ s, long long n, double *partial) {
     double m = 0;
@@ -62,20 +94,22 @@ __global__ void __launch_bounds__(OC_BS) k_oc_maxabs(const float *__restrict__ s
         for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
         if (threadIdx.x == 0) partial[4 + blockIdx.x] = m;
     }
-}
-
-__global__ void k_oc_init(double *st, int nb) {
+    if (!last_cta(partial)) return;
+    m = 0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) m = fmax(m, __ldcg(&partial[4 + b]));
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        double m = 0;
-        for (int b = 0; b < nb; b++) m = fmax(m, st[4 + b]);
-        st[0] = 0.0;
-        st[1] = (double)(float)m;
-        st[2] = 0.0;
+        for (int w = 1; w < OC_BS / 32; ++w) m = fmax(m, sm[w]);
+        partial[0] = 0.0;
+        partial[1] = (double)(float)m;
+        partial[2] = 0.0;
     }
 }
 
 __global__ void __launch_bounds__(OC_BS) k_oc_step(const float *__restrict__ sens, const float *__restrict__ rho,
-                                                   float *rho_new, long long n, float minrho, float step, float damp,
+                                                   float *rho_new, long long n, float vol, float minrho, float step, float damp,
                                                    double *st) {
     if (st[2] != 0.0) return;  // converged in an earlier step: keep its densities
     const float g = ((float)st[1] + (float)st[0]) / 2;
@@ -94,27 +128,22 @@ __global__ void __launch_bounds__(OC_BS) k_oc_step(const float *__restrict__ sen
     }
     double ss[1] = {s};
     block_reduce<1>(ss, st + 4, blockIdx.x);
-}
-
-__global__ void k_oc_decide(double *st, int nb, long long n, float vol) {
-    if (threadIdx.x != 0 || st[2] != 0.0) return;
-    double s = 0;
-    for (int b = 0; b < nb; b++) s += st[4 + b];
-    const float cur = (float)(s / (double)n);
-    const float g = ((float)st[1] + (float)st[0]) / 2;
-    if (cur < vol - 0.0001f) st[1] = g;
-    else if (cur > vol + 0.0001f) st[0] = g;
-    else st[2] = 1.0;
+    if (!last_cta(st)) return;
+    s = sum_partials(st, gridDim.x);
+    if (threadIdx.x == 0) {
+        const float cur = (float)(s / (double)n);
+        if (cur < vol - 0.0001f) st[1] = g;
+        else if (cur > vol + 0.0001f) st[0] = g;
+        else st[2] = 1.0;
+    }
 }
 
 void launch_oc(const float *sens, float *rho, float *rho_new, long long n, float vol, float minrho, float step,
                float damp, double *scratch, cudaStream_t s) {
+    cudaMemsetAsync(scratch, 0, 4 * sizeof(double), s);
     k_oc_maxabs<<<OC_NB, OC_BS, 0, s>>>(sens, n, scratch);
-    k_oc_init<<<1, 32, 0, s>>>(scratch, OC_NB);
-    for (int it = 0; it < 20; ++it) {
-        k_oc_step<<<OC_NB, OC_BS, 0, s>>>(sens, rho, rho_new, n, minrho, step, damp, scratch);
-        k_oc_decide<<<1, 32, 0, s>>>(scratch, OC_NB, n, vol);
-    }
+    for (int it = 0; it < 20; ++it)
+        k_oc_step<<<OC_NB, OC_BS, 0, s>>>(sens, rho, rho_new, n, vol, minrho, step, damp, scratch);
     cudaMemcpyAsync(rho, rho_new, sizeof(float) * n, cudaMemcpyDeviceToDevice, s);
 }
 
@@ -478,10 +507,10 @@ __global__ void __launch_bounds__(OC_BS) k_level_step(const float *__restrict__ 
     block_reduce<1>(ss, st + 4, blockIdx.x);
 }
 
-__global__ void k_level_decide(double *st, int nb, long long n, float vol) {
-    if (threadIdx.x != 0 || st[2] != 0.0) return;
-    double s = 0;
-    for (int b = 0; b < nb; b++) s += st[4 + b];
+__global__ void __launch_bounds__(OC_BS) k_level_decide(double *st, int nb, long long n, float vol) {
+    if (st[2] != 0.0) return;
+    const double s = sum_partials(st, nb);
+    if (threadIdx.x != 0) return;
     const float mean = (float)(s / (double)n);
     const float t = ((float)st[1] + (float)st[0]) / 2;
     st[3] = t;
@@ -517,7 +546,7 @@ int launch_trig_init(const int n[3], int P, const float *coeff_dev, int centered
     k_level_init<<<1, 32, 0, s>>>(scratch, (float)P);
     for (int it = 0; it < 60; ++it) {
         k_level_step<<<OC_NB, OC_BS, 0, s>>>(rho, ne, M, scratch);
-        k_level_decide<<<1, 32, 0, s>>>(scratch, OC_NB, ne, vol);
+        k_level_decide<<<1, OC_BS, 0, s>>>(scratch, OC_NB, ne, vol);
     }
     k_level_apply<<<OC_NB, OC_BS, 0, s>>>(rho, ne, M, scratch);
     return 0;

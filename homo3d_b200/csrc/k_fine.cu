@@ -838,24 +838,36 @@ void launch_rhs(const Level &L, const float *rho, const RhsTab &g, float *f, cud
 // ---- FP64 helpers of the refined mode ---------------------------------------------
 // u64 += e + T (T: the pending rigid translation of each of the 18 planes, see
 // k_pin_deflate); the pinned origin (colour 7, first vertex) keeps its value
-// Element-wise kernels over a blocked field run in storage order: one CTA of FVB
-// threads per (128-vertex block, plane) chunk c, plane q = c % 18, vertex
-// v = (c / 18) * FVB + thread (v >= nv in the padding of the last block).
-__device__ __forceinline__ void field_elem(long long &o, int &q, long long &v) {
-    const unsigned c = blockIdx.x;
-    q = (int)(c % NF);
-    v = (long long)(c / NF) * FVB + threadIdx.x;
-    o = (long long)c * FVB + threadIdx.x;
+// Element-wise kernels over a blocked field run in storage order, four values of one
+// plane per thread (128- and 256-bit accesses); vertices v >= nv are the padding of
+// the last block.  One value per thread ran at 2 to 4.7 TB/s.
+constexpr int FEB = 256;
+__device__ __forceinline__ bool field_quad(long long nv, long long &o, int &q, long long &v) {
+    const long long t = blockIdx.x * (long long)FEB + threadIdx.x;  // quad index
+    const long long c = t / (FVB / 4);                              // chunk: (vertex block, plane)
+    const long long b = c / NF;
+    q = (int)(c - b * NF);
+    v = b * FVB + (t - c * (FVB / 4)) * 4;
+    o = 4 * t;
+    return v < nv;
 }
-static unsigned field_chunks(long long nv) { return (unsigned)(field_floats(nv) / FVB); }
+static unsigned field_quad_blocks(long long nv) { return (unsigned)((field_floats(nv) / 4 + FEB - 1) / FEB); }
 
-__global__ void __launch_bounds__(FVB) k_update64(long long nv, double *u, const float *__restrict__ e,
+__global__ void __launch_bounds__(FEB) k_update64(long long nv, double *u, const float *__restrict__ e,
                                                  const double *__restrict__ T, long long pin) {
     long long o, v;
     int q;
-    field_elem(o, q, v);
-    if (v >= nv || v == pin) return;
-    u[o] += (double)e[o] + T[q];
+    if (!field_quad(nv, o, q, v)) return;
+    const float4 d = *reinterpret_cast<const float4 *>(e + o);
+    double2 *p = reinterpret_cast<double2 *>(u + o);
+    double2 a = p[0], b = p[1];
+    const double t = T[q];
+    if (v != pin) a.x += (double)d.x + t;
+    if (v + 1 < nv && v + 1 != pin) a.y += (double)d.y + t;
+    if (v + 2 < nv && v + 2 != pin) b.x += (double)d.z + t;
+    if (v + 3 < nv && v + 3 != pin) b.y += (double)d.w + t;
+    p[0] = a;
+    p[1] = b;
 }
 
 // ---- rigid-translation deflation of the pinned problem -------------------------
@@ -950,83 +962,99 @@ __global__ void k_pin_init(const double *__restrict__ sums, const float *__restr
     state[NF + i] = 0.0;
 }
 
-// FP32 solutions: u += T on every vertex but the origin (grid-stride)
-__global__ void k_pin_fold_u(long long nv, float *u, const double *__restrict__ state, long long pin) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv * NF;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long v = i % nv, q = i / nv;
-        if (v != pin) u[fidx((int)q, v)] = (float)((double)u[fidx((int)q, v)] + state[NF + q]);
-    }
+// FP32 solutions: u += T on every vertex but the origin
+__global__ void __launch_bounds__(FEB) k_pin_fold_u(long long nv, float *u, const double *__restrict__ state,
+                                                    long long pin) {
+    long long o, v;
+    int q;
+    if (!field_quad(nv, o, q, v)) return;
+    float4 *p = reinterpret_cast<float4 *>(u + o);
+    float4 a = *p;
+    const double t = state[NF + q];
+    if (v != pin) a.x = (float)((double)a.x + t);
+    if (v + 1 < nv && v + 1 != pin) a.y = (float)((double)a.y + t);
+    if (v + 2 < nv && v + 2 != pin) a.z = (float)((double)a.z + t);
+    if (v + 3 < nv && v + 3 != pin) a.w = (float)((double)a.w + t);
+    *p = a;
 }
 
-// undo the fold of T into f at the origin's neighbours, then T = 0
-__global__ void k_pin_restore_f(FineArgs a, const __grid_constant__ KeMat ke, double *state) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// undo the fold of T into f at the origin's neighbours, then T = 0; one thread per
+// (neighbour, case, component) as in k_pin_deflate (one thread for all: 130-180 us)
+__global__ void __launch_bounds__(PIN_THREADS) k_pin_restore_f(FineArgs a, const __grid_constant__ KeMat ke,
+                                                               double *state) {
+    __shared__ double T[NF];
+    const int tid = threadIdx.x, n = tid / NF, cr = tid % NF, c = cr / 3, r = cr % 3;
+    const int d = n < 13 ? n : n + 1;
+    if (tid < NF) T[tid] = state[NF + tid];
     const VertexGeo<7> g(a, 0);
-    for (int d = 0; d < 27; ++d) {
-        if (d == 13) continue;
-        int Kn;
-        bool pinned;
-        const unsigned nid = g.nbr(a, d, Kn, pinned);
-        if (pinned) continue;
-        float A[9];
-        g.block(ke, d, A);
-        for (int c = 0; c < NCASE; ++c)
-            for (int r = 0; r < 3; ++r) {
-                const double *T = state + NF + 3 * c;
-                const double t = (double)A[r] * T[0] + (double)A[3 + r] * T[1] + (double)A[6 + r] * T[2];
-                float *fp = const_cast<float *>(a.f) + fidx(3 * c + r, nid);
-                *fp = (float)((double)*fp - t);
-            }
-    }
-    for (int i = 0; i < NF; ++i) state[NF + i] = 0.0;
+    int Kn;
+    bool pinned;
+    const unsigned nid = g.nbr(a, d, Kn, pinned);
+    float A[9];
+    g.block(ke, d, A);
+    __syncthreads();
+    if (tid < NF) state[NF + tid] = 0.0;
+    if (pinned) return;
+    const double t = (double)A[r] * T[3 * c] + (double)A[3 + r] * T[3 * c + 1] + (double)A[6 + r] * T[3 * c + 2];
+    float *fp = const_cast<float *>(a.f) + fidx(3 * c + r, nid);
+    *fp = (float)((double)*fp - t);
 }
 
-// FP32 field <-> FP64 field (both blocked)
-__global__ void __launch_bounds__(FVB) k_f32_to_f64(long long nv, const float *__restrict__ s, double *d) {
+// FP32 field <-> FP64 field (both blocked; the padding holds whatever it held)
+__global__ void __launch_bounds__(FEB) k_f32_to_f64(long long nv, const float *__restrict__ s, double *d) {
     long long o, v;
     int q;
-    field_elem(o, q, v);
-    if (v < nv) d[o] = (double)s[o];
+    if (!field_quad(nv, o, q, v)) return;
+    const float4 a = *reinterpret_cast<const float4 *>(s + o);
+    double2 *p = reinterpret_cast<double2 *>(d + o);
+    p[0] = make_double2((double)a.x, (double)a.y);
+    p[1] = make_double2((double)a.z, (double)a.w);
 }
 
-__global__ void __launch_bounds__(FVB) k_f64_to_f32(long long nv, const double *__restrict__ s, float *d) {
+__global__ void __launch_bounds__(FEB) k_f64_to_f32(long long nv, const double *__restrict__ s, float *d) {
     long long o, v;
     int q;
-    field_elem(o, q, v);
-    if (v < nv) d[o] = (float)s[o];
+    if (!field_quad(nv, o, q, v)) return;
+    const double2 *p = reinterpret_cast<const double2 *>(s + o);
+    const double2 a = p[0], b = p[1];
+    *reinterpret_cast<float4 *>(d + o) = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
 }
 
 void launch_update64(const Level &L, double *u64, const float *e, const double *T, cudaStream_t s) {
-    k_update64<<<field_chunks(L.P.nv), FVB, 0, s>>>(L.P.nv, u64, e, T, L.P.base[7]);
+    k_update64<<<field_quad_blocks(L.P.nv), FEB, 0, s>>>(L.P.nv, u64, e, T, L.P.base[7]);
 }
 void launch_pin_deflate(const Level &L, const float *rho, const KeMat &ke, double *state, cudaStream_t s) {
     k_pin_deflate<<<1, PIN_THREADS, 0, s>>>(make_args(L, rho), ke, state);
 }
 // level-0 f of a zero FP64 solution: f0 - K 0 = f0 on every vertex but the pinned
 // origin, whose residual is 0 (what k_fine_residual64 computes for u64 = 0)
-__global__ void __launch_bounds__(FVB) k_rhs_at_zero(long long nv, const float *__restrict__ f0, float *f,
+__global__ void __launch_bounds__(FEB) k_rhs_at_zero(long long nv, const float *__restrict__ f0, float *f,
                                                     long long pin) {
     long long o, v;
     int q;
-    field_elem(o, q, v);
-    if (v < nv) f[o] = v == pin ? 0.f : f0[o];
+    if (!field_quad(nv, o, q, v)) return;
+    float4 a = *reinterpret_cast<const float4 *>(f0 + o);
+    if (v == pin) a.x = 0.f;
+    else if (v + 1 == pin) a.y = 0.f;
+    else if (v + 2 == pin) a.z = 0.f;
+    else if (v + 3 == pin) a.w = 0.f;
+    *reinterpret_cast<float4 *>(f + o) = a;
 }
 void launch_rhs_at_zero(const Level &L, const float *f0, float *f, cudaStream_t s) {
-    k_rhs_at_zero<<<field_chunks(L.P.nv), FVB, 0, s>>>(L.P.nv, f0, f, L.P.base[7]);
+    k_rhs_at_zero<<<field_quad_blocks(L.P.nv), FEB, 0, s>>>(L.P.nv, f0, f, L.P.base[7]);
 }
 void launch_pin_init(const Level &L, const double *sums, double *state, cudaStream_t s) {
     k_pin_init<<<1, 32, 0, s>>>(sums, L.f, L.P.nv, L.P.base[7], state);
 }
 void launch_pin_fold(const Level &L, const float *rho, const KeMat &ke, double *state, cudaStream_t s) {
-    k_pin_fold_u<<<1184, 256, 0, s>>>(L.P.nv, L.u, state, L.P.base[7]);
-    k_pin_restore_f<<<1, 32, 0, s>>>(make_args(L, rho), ke, state);
+    k_pin_fold_u<<<field_quad_blocks(L.P.nv), FEB, 0, s>>>(L.P.nv, L.u, state, L.P.base[7]);
+    k_pin_restore_f<<<1, PIN_THREADS, 0, s>>>(make_args(L, rho), ke, state);
 }
 void launch_convert_field(long long nv, const float *src, double *dst, cudaStream_t s) {
-    k_f32_to_f64<<<field_chunks(nv), FVB, 0, s>>>(nv, src, dst);
+    k_f32_to_f64<<<field_quad_blocks(nv), FEB, 0, s>>>(nv, src, dst);
 }
 void launch_convert_field(long long nv, const double *src, float *dst, cudaStream_t s) {
-    k_f64_to_f32<<<field_chunks(nv), FVB, 0, s>>>(nv, src, dst);
+    k_f64_to_f32<<<field_quad_blocks(nv), FEB, 0, s>>>(nv, src, dst);
 }
 
 // ---- lockstep batches: the level 0 of several designs in one launch per step ----
