@@ -37,10 +37,12 @@ def _spline(q):
     return 1 - 6 * q + 8 * q ** 1.5 - 3 * q * q if q < 1 else 0.0
 
 
-# windows of one cell, of 3, 5 and 9 cells, on a grid narrower than a block of threads,
-# one with a partial block in x and y, and one where only the window's middle is whole
-@pytest.mark.parametrize("n,radius,periodic", [(10, 0.4, True), (10, 1.2, False), (40, 2.0, True), (40, 2.0, False),
-                                               (20, 4.3, True), (12, 4.3, False)])
+# windows of 1, 3, 5, 7, 9 and 11 cells (the first and last run cell by cell), on a grid
+# narrower than a block of threads and with a partial column of four cells (10), one with
+# a partial block in x and y (40), and ones where few or no windows are whole (12)
+@pytest.mark.parametrize("n,radius,periodic", [(10, 0.4, True), (10, 1.2, False), (10, 2.6, True), (40, 2.0, True),
+                                               (40, 2.0, False), (20, 2.6, False), (20, 4.3, True), (12, 4.3, False),
+                                               (20, 5.2, True), (12, 5.2, False)])
 def test_window_sums(torch_cuda, n, radius, periodic):
     torch = torch_cuda
     hd = H.Homogenization(n)
