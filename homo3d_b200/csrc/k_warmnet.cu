@@ -31,99 +31,159 @@
 namespace h3d {
 
 constexpr int WN_BS = 128;
-constexpr int WN_CO = 8;  // output channels per thread in the convolution kernels
+constexpr int WN_CI = 16;  // input channels whose weights are staged at a time
 
 __device__ __forceinline__ int wn_wrap(int a, int r) { return a < 0 ? a + r : (a >= r ? a - r : a); }
+
+// indices of the 27 neighbours of voxel v (offsets negated for s = -1)
+__device__ __forceinline__ void wn_nbrs(int v, int R, int s, int nb[27]) {
+    const int vx = v % R, vy = (v / R) % R, vz = v / (R * R);
+    int X[3], Y[3], Z[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        X[d] = wn_wrap(vx + s * (d - 1), R);
+        Y[d] = R * wn_wrap(vy + s * (d - 1), R);
+        Z[d] = R * R * wn_wrap(vz + s * (d - 1), R);
+    }
+#pragma unroll
+    for (int t = 0; t < 27; ++t) nb[t] = X[t % 3] + Y[t / 3 % 3] + Z[t / 9];
+}
 
 // y[b][co][v] = bias[co] + sum_ci sum_t W[co][ci][t] x[b][ci][v + off(t)], then
 // optionally ReLU.  TRANSPOSED computes the input gradient of a convolution:
 // dx[b][ci][v] = sum_co sum_t W[co][ci][t] dy[b][co][v - off(t)] (the kernel's
 // input channels are the convolution's outputs; taps mirrored; no bias).
-template <bool TRANSPOSED>
+// A thread forms CO output channels of one voxel; the weights of WN_CI input channels
+// are staged in shared memory as [ci][t][co], so a tap is one or two vector loads and CO
+// FMAs.  Reading each weight from global memory, one load per FMA, was bound by the
+// load/store pipe (0.14 ms per layer of the 32^3 network, batch 4; 0.05 ms now).  CO is 8, or 4 or 2
+// where a level's voxels alone leave the chip idle (wn_conv).
+template <bool TRANSPOSED, int CO>
 __global__ void __launch_bounds__(WN_BS) k_wn_conv3(const float *__restrict__ x, const float *__restrict__ W,
                                                    const float *__restrict__ bias, float *y, int Cin, int Cout, int R,
                                                    int relu) {
+    __shared__ __align__(16) float ws[WN_CI * 27 * CO];
     const int R3 = R * R * R;
-    const int v = blockIdx.x * WN_BS + threadIdx.x;
-    const int co0 = blockIdx.y * WN_CO, b = blockIdx.z;
-    if (v >= R3) return;
-    const int vx = v % R, vy = (v / R) % R, vz = v / (R * R);
-    const int s = TRANSPOSED ? -1 : 1;
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    const int co0 = blockIdx.y * CO, b = blockIdx.z;
+    const bool on = v < R3;
     int nb[27];
+    wn_nbrs(on ? v : 0, R, TRANSPOSED ? -1 : 1, nb);
+    float acc[CO];
 #pragma unroll
-    for (int t = 0; t < 27; ++t) {
-        const int dx = t % 3 - 1, dy = t / 3 % 3 - 1, dz = t / 9 - 1;
-        nb[t] = wn_wrap(vx + s * dx, R) + R * (wn_wrap(vy + s * dy, R) + R * wn_wrap(vz + s * dz, R));
-    }
-    float acc[WN_CO];
-#pragma unroll
-    for (int q = 0; q < WN_CO; ++q) acc[q] = (!TRANSPOSED && bias && co0 + q < Cout) ? bias[co0 + q] : 0.f;
+    for (int q = 0; q < CO; ++q) acc[q] = (!TRANSPOSED && bias && co0 + q < Cout) ? bias[co0 + q] : 0.f;
     const float *xb = x + (long long)b * Cin * R3;
-    for (int ci = 0; ci < Cin; ++ci) {
-        const float *xc = xb + (long long)ci * R3;
-        float in[27];
+    for (int c0 = 0; c0 < Cin; c0 += WN_CI) {
+        const int nc = min(WN_CI, Cin - c0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < nc * 27 * CO; i += blockDim.x) {
+            const int ci = c0 + i / (27 * CO), t = i / CO % 27, co = co0 + i % CO;
+            ws[i] = co >= Cout ? 0.f
+                  : __ldg(TRANSPOSED ? W + ((long long)ci * Cout + co) * 27 + t : W + ((long long)co * Cin + ci) * 27 + t);
+        }
+        __syncthreads();
+        if (!on) continue;
+        for (int c = 0; c < nc; ++c) {
+            const float *xc = xb + (long long)(c0 + c) * R3;
+            const float *wc = ws + c * 27 * CO;
+            float in[27];
 #pragma unroll
-        for (int t = 0; t < 27; ++t) in[t] = __ldg(xc + nb[t]);
+            for (int t = 0; t < 27; ++t) in[t] = __ldg(xc + nb[t]);
 #pragma unroll
-        for (int q = 0; q < WN_CO; ++q) {
-            const int co = co0 + q;
-            if (co < Cout) {
-                const float *w = TRANSPOSED ? W + ((long long)ci * Cout + co) * 27 : W + ((long long)co * Cin + ci) * 27;
-                float a = acc[q];
+            for (int t = 0; t < 27; ++t) {
+                float w[CO];
+                if (CO == 2) {
+                    *reinterpret_cast<float2 *>(w) = *reinterpret_cast<const float2 *>(wc + t * CO);
+                } else {
 #pragma unroll
-                for (int t = 0; t < 27; ++t) a = fmaf(__ldg(w + t), in[t], a);
-                acc[q] = a;
+                    for (int q = 0; q < CO; q += 4)
+                        *reinterpret_cast<float4 *>(w + q) = *reinterpret_cast<const float4 *>(wc + t * CO + q);
+                }
+#pragma unroll
+                for (int q = 0; q < CO; ++q) acc[q] = fmaf(w[q], in[t], acc[q]);
             }
         }
     }
+    if (!on) return;
     float *yb = y + (long long)b * Cout * R3;
 #pragma unroll
-    for (int q = 0; q < WN_CO; ++q) {
+    for (int q = 0; q < CO; ++q) {
         const int co = co0 + q;
         if (co < Cout) yb[(long long)co * R3 + v] = relu ? fmaxf(acc[q], 0.f) : acc[q];
     }
 }
 
-// dW[co][ci][t] += sum_b sum_v dz[b][co][v] x[b][ci][v + off(t)], and for ci == 0
-// db[co] += sum dz[b][co][v]; one block per (co, ci), fixed-order reduction
-__global__ void __launch_bounds__(WN_BS) k_wn_conv3_wgrad(const float *__restrict__ x, const float *__restrict__ dz,
-                                                         float *dW, float *db, int Cin, int Cout, int R, int B) {
-    const int co = blockIdx.x / Cin, ci = blockIdx.x % Cin;
-    const int R3 = R * R * R;
-    float g[28];
-#pragma unroll
-    for (int t = 0; t < 28; ++t) g[t] = 0.f;
-    for (int b = 0; b < B; ++b) {
-        const float *xc = x + ((long long)b * Cin + ci) * R3;
-        const float *dc = dz + ((long long)b * Cout + co) * R3;
-        for (int v = threadIdx.x; v < R3; v += WN_BS) {
-            const int vx = v % R, vy = (v / R) % R, vz = v / (R * R);
-            const float d = __ldg(dc + v);
-#pragma unroll
-            for (int t = 0; t < 27; ++t) {
-                const int dx = t % 3 - 1, dy = t / 3 % 3 - 1, dzz = t / 9 - 1;
-                const int n = wn_wrap(vx + dx, R) + R * (wn_wrap(vy + dy, R) + R * wn_wrap(vz + dzz, R));
-                g[t] = fmaf(d, __ldg(xc + n), g[t]);
-            }
-            g[27] += d;
-        }
-    }
-    __shared__ float red[28][WN_BS / 32];
+// sums of N values per thread over the CTA, value i to out[i] (fixed order)
+template <int N>
+__device__ __forceinline__ void wn_cta_sums(const float *g, float *out) {
+    __shared__ float red[N][WN_BS / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int t = 0; t < 28; ++t) {
+    for (int t = 0; t < N; ++t) {
         float v = g[t];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) red[t][wid] = v;
     }
     __syncthreads();
-    if (threadIdx.x < 28) {
+    for (int t = threadIdx.x; t < N; t += WN_BS) {
         float v = 0.f;
-        for (int w = 0; w < WN_BS / 32; ++w) v += red[threadIdx.x][w];
-        if (threadIdx.x < 27) dW[((long long)co * Cin + ci) * 27 + threadIdx.x] += v;
-        else if (ci == 0) db[co] += v;
+#pragma unroll
+        for (int w = 0; w < WN_BS / 32; ++w) v += red[t][w];
+        out[t] = v;
     }
+}
+
+// Weight gradients, dW[co][ci][t] += sum_b sum_v dz[b][co][v] x[b][ci][v + off(t)] and
+// db[co] += sum dz[b][co][v], in two stages: CTA (co group, ci, chunk) sums its chunk of
+// the batch's voxels for WN_GCO output channels (27 x values and WN_GCO dz values for
+// 27 WN_GCO FMAs), k_wn_grad_finish adds the chunks in order.  One CTA per (co, ci)
+// over all voxels left most of the chip idle and loaded a value per FMA: 0.33 ms per
+// layer of the 32^3 network, batch 4; 0.06 ms now.
+constexpr int WN_GCO = 4;
+constexpr int WN_GROW = 28 * WN_GCO;  // partial row: [WN_GCO][27 taps, bias]
+__global__ void __launch_bounds__(WN_BS) k_wn_conv3_wgrad(const float *__restrict__ x, const float *__restrict__ dz,
+                                                         float *part, int Cin, int Cout, int R, int B, int chunk) {
+    const int ci = blockIdx.x % Cin, co0 = blockIdx.x / Cin * WN_GCO;
+    const int R3 = R * R * R, n = B * R3;
+    const int i0 = blockIdx.y * chunk, i1 = min(n, i0 + chunk);
+    float g[WN_GROW];
+#pragma unroll
+    for (int t = 0; t < WN_GROW; ++t) g[t] = 0.f;
+    for (int i = i0 + threadIdx.x; i < i1; i += WN_BS) {
+        const int b = i / R3, v = i - b * R3;
+        const float *xc = x + ((long long)b * Cin + ci) * R3;
+        const float *dc = dz + ((long long)b * Cout + co0) * R3 + v;
+        int nb[27];
+        wn_nbrs(v, R, 1, nb);
+        float d[WN_GCO];
+#pragma unroll
+        for (int q = 0; q < WN_GCO; ++q) {
+            d[q] = __ldg(dc + (long long)q * R3);
+            g[28 * q + 27] += d[q];
+        }
+#pragma unroll
+        for (int t = 0; t < 27; ++t) {
+            const float a = __ldg(xc + nb[t]);
+#pragma unroll
+            for (int q = 0; q < WN_GCO; ++q) g[28 * q + t] = fmaf(d[q], a, g[28 * q + t]);
+        }
+    }
+    wn_cta_sums<WN_GROW>(g, part + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * WN_GROW);
+}
+
+// one thread per weight (and, for ci = 0, bias): the chunks' partial sums in order
+__global__ void __launch_bounds__(WN_BS) k_wn_grad_finish(const float *__restrict__ part, float *dW, float *db, int Cin,
+                                                         int Cout, int nchunk) {
+    const int i = blockIdx.x * WN_BS + threadIdx.x, nrow = Cout / WN_GCO * Cin;
+    if (i >= nrow * WN_GROW) return;
+    const int row = i / WN_GROW, e = i % WN_GROW, t = e % 28;
+    const int ci = row % Cin, co = row / Cin * WN_GCO + e / 28;
+    if (t == 27 && ci != 0) return;
+    float v = 0.f;
+    for (int k = 0; k < nchunk; ++k) v += __ldg(part + ((long long)k * nrow) * WN_GROW + i);
+    if (t < 27) dW[((long long)co * Cin + ci) * 27 + t] += v;
+    else db[co] += v;
 }
 
 // 1x1 output layer: y[b][o][v] = bias[o] + sum_c W[o][c] x[b][c][v]
@@ -155,27 +215,44 @@ __global__ void k_wn_out_bwd(const float *__restrict__ dy, const float *__restri
     }
 }
 
-// weight gradient of the 1x1 layer: one block per (o, c), c == Cin for the bias
+// weight gradient of the 1x1 layer (16 inputs): CTA (group of WN_OG outputs, chunk) sums
+// its chunk for WN_OG x (16 weights, bias); k_wn_out_finish adds the chunks in order
+constexpr int WN_OG = 6, WN_OIN = 16, WN_OROW = WN_OG * (WN_OIN + 1);
 __global__ void __launch_bounds__(WN_BS) k_wn_out_wgrad(const float *__restrict__ x, const float *__restrict__ dy,
-                                                       float *dW, float *db, int Cin, int Cout, int R3, int B) {
-    const int o = blockIdx.x / (Cin + 1), c = blockIdx.x % (Cin + 1);
-    float s = 0.f;
-    for (int b = 0; b < B; ++b)
-        for (int v = threadIdx.x; v < R3; v += WN_BS) {
-            const float d = dy[((long long)b * Cout + o) * R3 + v];
-            s = fmaf(d, c < Cin ? x[((long long)b * Cin + c) * R3 + v] : 1.f, s);
-        }
-    __shared__ float red[WN_BS / 32];
+                                                       float *part, int Cout, int R3, int B, int chunk) {
+    const int o0 = blockIdx.x * WN_OG, n = B * R3;
+    const int i0 = blockIdx.y * chunk, i1 = min(n, i0 + chunk);
+    float g[WN_OROW];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float v = 0.f;
-        for (int w = 0; w < WN_BS / 32; ++w) v += red[w];
-        if (c < Cin) dW[o * Cin + c] += v;
-        else db[o] += v;
+    for (int t = 0; t < WN_OROW; ++t) g[t] = 0.f;
+    for (int i = i0 + threadIdx.x; i < i1; i += WN_BS) {
+        const int b = i / R3, v = i - b * R3;
+        const float *xb = x + (long long)b * WN_OIN * R3 + v, *db = dy + ((long long)b * Cout + o0) * R3 + v;
+        float d[WN_OG];
+#pragma unroll
+        for (int q = 0; q < WN_OG; ++q) {
+            d[q] = __ldg(db + (long long)q * R3);
+            g[q * (WN_OIN + 1) + WN_OIN] += d[q];
+        }
+#pragma unroll
+        for (int c = 0; c < WN_OIN; ++c) {
+            const float a = __ldg(xb + (long long)c * R3);
+#pragma unroll
+            for (int q = 0; q < WN_OG; ++q) g[q * (WN_OIN + 1) + c] = fmaf(d[q], a, g[q * (WN_OIN + 1) + c]);
+        }
     }
+    wn_cta_sums<WN_OROW>(g, part + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * WN_OROW);
+}
+
+__global__ void __launch_bounds__(WN_BS) k_wn_out_finish(const float *__restrict__ part, float *dW, float *db, int Cout,
+                                                        int nchunk) {
+    const int i = blockIdx.x * WN_BS + threadIdx.x, n = Cout * (WN_OIN + 1);
+    if (i >= n) return;
+    float v = 0.f;
+    for (int k = 0; k < nchunk; ++k) v += __ldg(part + (long long)k * n + i);
+    const int o = i / (WN_OIN + 1), c = i % (WN_OIN + 1);
+    if (c < WN_OIN) dW[o * WN_OIN + c] += v;
+    else db[o] += v;
 }
 
 // dz = dy * (y > 0), in place on dy
@@ -324,6 +401,12 @@ constexpr int WN_NCONV = 7;
 constexpr int WN_LAYER[WN_NCONV][3] = {{1, 16, 0}, {16, 32, 1}, {32, 64, 2}, {64, 64, 3},
                                        {64, 32, 2}, {32, 16, 1}, {16, 16, 0}};
 constexpr int WN_OUT_IN = 16, WN_OUT = NF;
+static_assert(WN_OUT_IN == WN_OIN && WN_OUT % WN_OG == 0, "the 1x1 layer's gradient kernel");
+// scratch of the weight gradients: the chunks' partial sums (grad_chunks keeps rows x
+// chunks at or below 1184 rows more than one chunk's)
+constexpr int WN_MAXCHUNK = 512;
+constexpr long long WN_GPART = (1184ll + 64 / WN_GCO * 64) * WN_GROW;
+static_assert(WN_GPART >= (long long)WN_MAXCHUNK * NF * (WN_OIN + 1), "the 1x1 layer's partial sums");
 
 }  // namespace
 
@@ -337,6 +420,7 @@ struct h3d_warmnet {
     float *a0, *p1, *a1, *p2, *a2, *p3, *a3, *u2, *d2, *u1, *d1, *u0, *d0, *y;
     float *ga0, *gp1, *ga1, *gp2, *ga2, *gp3, *ga3, *gu2, *gd2, *gu1, *gd1, *gu0, *gd0, *gy;
     float *act = nullptr;
+    float *gpart = nullptr;  // partial weight gradients
     double *partial = nullptr, *d_loss = nullptr, *h_loss = nullptr;
     long long step = 0;
     std::string err;
@@ -366,22 +450,46 @@ uint64_t splitmix(uint64_t &s) {
     return z ^ (z >> 31);
 }
 
+// output channels per thread: 8, fewer while the launch has fewer than two CTAs per SM
+template <bool TRANSPOSED>
+void wn_conv(const float *x, const float *W, const float *bias, float *y, int cin, int cout, int R, int relu, int B,
+             cudaStream_t s) {
+    const long long v = (long long)R * R * R;
+    const unsigned nt = v <= 64 ? 64 : WN_BS, nv = nblk(v, nt);
+    int co = 8;
+    while (co > 2 && (long long)nv * ((cout + co - 1) / co) * B < 296) co /= 2;
+    const dim3 grid(nv, (cout + co - 1) / co, B);
+    if (co == 8) k_wn_conv3<TRANSPOSED, 8><<<grid, nt, 0, s>>>(x, W, bias, y, cin, cout, R, relu);
+    else if (co == 4) k_wn_conv3<TRANSPOSED, 4><<<grid, nt, 0, s>>>(x, W, bias, y, cin, cout, R, relu);
+    else k_wn_conv3<TRANSPOSED, 2><<<grid, nt, 0, s>>>(x, W, bias, y, cin, cout, R, relu);
+}
+
 void conv(h3d_warmnet *n, int layer, const float *x, float *y, int B, cudaStream_t s) {
     const int ci = WN_LAYER[layer][0], co = WN_LAYER[layer][1], R = n->lvl(WN_LAYER[layer][2]);
-    const dim3 grid(nblk((long long)R * R * R, WN_BS), (co + WN_CO - 1) / WN_CO, B);
-    k_wn_conv3<false><<<grid, WN_BS, 0, s>>>(x, n->w + n->woff[layer], n->w + n->boff[layer], y, ci, co, R, 1);
+    wn_conv<false>(x, n->w + n->woff[layer], n->w + n->boff[layer], y, ci, co, R, 1, B, s);
 }
 
 // input gradient of convolution `layer` from its (ReLU-masked) output gradient gz
 void conv_bwd_data(h3d_warmnet *n, int layer, const float *gz, float *gx, int B, cudaStream_t s) {
     const int ci = WN_LAYER[layer][0], co = WN_LAYER[layer][1], R = n->lvl(WN_LAYER[layer][2]);
-    const dim3 grid(nblk((long long)R * R * R, WN_BS), (ci + WN_CO - 1) / WN_CO, B);
-    k_wn_conv3<true><<<grid, WN_BS, 0, s>>>(gz, n->w + n->woff[layer], nullptr, gx, co, ci, R, 0);
+    wn_conv<true>(gz, n->w + n->woff[layer], nullptr, gx, co, ci, R, 0, B, s);
+}
+
+// chunks of `total` voxels for `rows` CTAs each: about eight CTAs per SM, no chunk below
+// 512 voxels (four per thread, against the cost of a CTA's sums)
+int grad_chunks(long long total, int rows) {
+    const long long most = (total + 511) / 512, want = (1184 + rows - 1) / rows;
+    return (int)std::max(1ll, std::min(most, std::min(want, (long long)WN_MAXCHUNK)));
 }
 
 void conv_wgrad(h3d_warmnet *n, int layer, const float *x, const float *gz, int B, cudaStream_t s) {
     const int ci = WN_LAYER[layer][0], co = WN_LAYER[layer][1], R = n->lvl(WN_LAYER[layer][2]);
-    k_wn_conv3_wgrad<<<co * ci, WN_BS, 0, s>>>(x, gz, n->g + n->woff[layer], n->g + n->boff[layer], ci, co, R, B);
+    const long long total = (long long)B * R * R * R;
+    const int rows = co / WN_GCO * ci, nc = grad_chunks(total, rows);
+    const int chunk = (int)((total + nc - 1) / nc);
+    k_wn_conv3_wgrad<<<dim3(rows, nc), WN_BS, 0, s>>>(x, gz, n->gpart, ci, co, R, B, chunk);
+    k_wn_grad_finish<<<nblk((long long)rows * WN_GROW, WN_BS), WN_BS, 0, s>>>(n->gpart, n->g + n->woff[layer],
+                                                                            n->g + n->boff[layer], ci, co, nc);
 }
 
 void relu_bwd(float *g, const float *y, long long cnt, cudaStream_t s) {
@@ -415,8 +523,11 @@ int backward(h3d_warmnet *n, const float *x, const float *t, int B, cudaStream_t
     const int nb = 256;
     k_wn_mse<<<nb, 256, 0, s>>>(n->y, t, n->gy, ny, n->partial);
     k_wn_sum<<<1, 32, 0, s>>>(n->partial, nb, n->d_loss, 1.0 / (double)ny);
-    k_wn_out_wgrad<<<WN_OUT * (WN_OUT_IN + 1), WN_BS, 0, s>>>(n->d0, n->gy, n->g + n->woff[WN_NCONV],
-                                                             n->g + n->boff[WN_NCONV], WN_OUT_IN, WN_OUT, (int)V0, B);
+    const int onc = grad_chunks(b * V0, WN_OUT / WN_OG);
+    k_wn_out_wgrad<<<dim3(WN_OUT / WN_OG, onc), WN_BS, 0, s>>>(n->d0, n->gy, n->gpart, WN_OUT, (int)V0, B,
+                                                             (int)((b * V0 + onc - 1) / onc));
+    k_wn_out_finish<<<nblk(WN_OUT * (WN_OIN + 1), WN_BS), WN_BS, 0, s>>>(n->gpart, n->g + n->woff[WN_NCONV],
+                                                                       n->g + n->boff[WN_NCONV], WN_OUT, onc);
     k_wn_out_bwd<<<nblk(b * V0, 128), 128, 0, s>>>(n->gy, n->w + n->woff[WN_NCONV], n->d0, n->gd0, WN_OUT_IN, WN_OUT,
                                                   (int)V0, B);
     // d0 = relu(conv6(u0)), u0 = up(d1) + a0
@@ -525,6 +636,7 @@ int h3d_warmnet_create(int reso, int max_batch, uint64_t seed, int device, h3d_w
     float *p = n->act;
     for (int i = 0; i < 14; i++) { *fw[i] = p; p += B * sizes[i]; }
     for (int i = 0; i < 14; i++) { *bw[i] = p; p += B * sizes[i]; }
+    if (cudaMalloc(&n->gpart, sizeof(float) * WN_GPART) != cudaSuccess) return bail(H3D_ERR_NOMEM);
     if (cudaMalloc(&n->partial, sizeof(double) * 256) != cudaSuccess) return bail(H3D_ERR_NOMEM);
     if (cudaMalloc(&n->d_loss, sizeof(double)) != cudaSuccess) return bail(H3D_ERR_NOMEM);
     if (cudaMallocHost(&n->h_loss, sizeof(double)) != cudaSuccess) return bail(H3D_ERR_NOMEM);
@@ -555,6 +667,7 @@ int h3d_warmnet_destroy(h3d_warmnet *n) {
     if (n->stream) cudaStreamSynchronize(n->stream);
     cudaFree(n->w);
     cudaFree(n->act);
+    cudaFree(n->gpart);
     cudaFree(n->partial);
     cudaFree(n->d_loss);
     cudaFreeHost(n->h_loss);
