@@ -305,10 +305,7 @@ int enqueue_vcycle(h3d_handle *h, float w, bool deflate = false) {
                 return fail(h, H3D_ERR_CUDA, "cooperative V-cycle bottom could not be launched");
             break;
         }
-        if (l > 0) {
-            launch_restrict(h->lv[l - 1], h->lv[l], s);
-            cudaMemsetAsync(h->lv[l].u, 0, sizeof(float) * field_floats(h->lv[l].P.nv), s);
-        }
+        if (l > 0) launch_restrict(h->lv[l - 1], h->lv[l], s);
         if (l == h->nl - 1) {
             launch_coarse_apply(h->lv[l], h->aug, h->cfg.coarse_mode == H3D_COARSE_PROJECT, s);
         } else if (l == 0 && h->mixed()) {  // the sweep, then the residual on the tensor cores
@@ -317,7 +314,7 @@ int enqueue_vcycle(h3d_handle *h, float w, bool deflate = false) {
         } else if (l == 0) {
             launch_fine_gs_residual(h->lv[0], h->rho, h->ke, w, h->partial, s);
         } else {
-            launch_coarse_gs_residual(h->lv[l], w, s);  // each level's residual comes with its sweep
+            launch_coarse_down(h->lv[l], w, s);  // from a zero correction
         }
     }
     for (int l = (bfirst >= 0 ? bfirst : h->nl - 1) - 1; l >= 0; l--) {
@@ -1296,7 +1293,7 @@ int h3d_batch_elastic_matrix(h3d_handle *const *hs, int n, double tol, double *C
 
 // ---- lockstep batches -------------------------------------------------------
 // The V-cycle of enqueue_vcycle for all designs at once: level index l runs, for
-// the designs that have it, the restriction into l (clearing l's solution), then
+// the designs that have it, the restriction into l, then
 // the down leg's sweep and residual, or the coarsest solve where l is a design's
 // last level; the up leg prolongs and sweeps; then the deflation and the norms.
 // Each design sees its own launches' operations in its own order.

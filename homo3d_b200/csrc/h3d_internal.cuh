@@ -321,9 +321,9 @@ void launch_remove_mean64(const Planes &P, double *v, double *partial, int nblk,
 // coarse levels and transfers (k_coarse.cu)
 void launch_coarse_gs(const Level &L, float w, cudaStream_t s);
 void launch_coarse_residual(const Level &L, cudaStream_t s);
-// a coarse colour sweep followed by the level's residual (the last colour's launch
-// computes its own vertices' residual)
-void launch_coarse_gs_residual(const Level &L, float w, cudaStream_t s);
+// the down leg of a coarse level: a colour sweep from u = 0 (u need not be cleared)
+// and the level's residual
+void launch_coarse_down(const Level &L, float w, cudaStream_t s);
 void launch_restrict(const Level &F, const Level &C, cudaStream_t s);
 void launch_prolong(const Level &F, const Level &C, int is_root, cudaStream_t s);
 void launch_weighted_norm(const Planes &P, const float *v, double *partial, int nblk, cudaStream_t s);
@@ -430,13 +430,13 @@ void launch_fine_sweep_batch(const BatchTab &t, const KeMat &ke, const int *acti
                              cudaStream_t s);
 void launch_pin_deflate_batch(const BatchTab &t, const KeMat &ke, const int *active, cudaStream_t s);
 // one coarse level of each design (all with the same stencil precision): the
-// sweep (launch shape 0: two cases per thread, 1: six), with residual the down
-// leg's sweep and residual; scratch as for level 0
+// sweep (launch shape 0: two cases per thread, 1: six), or the down leg's sweep from
+// u = 0 and residual; scratch as for level 0
 int coarse_batch_create(const Level *const *lv, const int *design, int n, bool scratch, BatchTab *out);
-void launch_coarse_sweep_batch(const BatchTab &t, bool f32, const int *active, bool residual, int shape,
+void launch_coarse_sweep_batch(const BatchTab &t, bool f32, const int *active, bool down, int shape,
                                cudaStream_t s);
 // ratio-2 transfers between levels F[i] (even) and C[i]: restriction of F.r into
-// C.f with C.u cleared, prolongation of C.u into F.u (is_root: F is level 0)
+// C.f, prolongation of C.u into F.u (is_root: F is level 0)
 int transfer_batch_create(const Level *const *F, const Level *const *C, const int *design, int n, BatchTab *out);
 void launch_restrict_batch(const BatchTab &t, const int *active, cudaStream_t s);
 void launch_prolong_batch(const BatchTab &t, const int *active, int is_root, cudaStream_t s);

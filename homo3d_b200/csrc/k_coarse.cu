@@ -67,7 +67,8 @@ __device__ __forceinline__ void load_block(const CoarseArgs &a, long long me, fl
 // colours)
 // CG: neighbour values through L2 only (ld.global.cg), for kernels that read values
 // other CTAs wrote earlier in the same launch
-template <int KC, bool SELF, bool F32, int C, bool CG = false>
+// PART: all neighbours, or those of the colours before (-1) or after (1) the vertex's
+template <int KC, bool SELF, bool F32, int C, bool CG = false, int PART = 0>
 __device__ __forceinline__ void coarse_apply(const CoarseArgs &a, long long me, int i, int j, int l, int cb,
                                              float acc[3 * C], int kr = KC) {
     static_assert(C % 2 == 0, "the load cases of a thread go in packed FP32x2 lane pairs");
@@ -96,6 +97,8 @@ __device__ __forceinline__ void coarse_apply(const CoarseArgs &a, long long me, 
     for (int d = 0; d < 27; ++d) {
         if (d == 13 && !SELF) continue;
         const int dx = d % 3 - 1, dy = d / 3 % 3 - 1, dz = d / 9 - 1;
+        const int Kn = K ^ ((dx & 1) | ((dy & 1) << 1) | ((dz & 1) << 2));
+        if ((PART < 0 && Kn > K) || (PART > 0 && Kn < K)) continue;
         float s[9];
         switch (d) {  // compile-time block index for the chunk arithmetic
 #define H3D_LB(D) case D: load_block<D, F32>(a, me, s); break;
@@ -105,7 +108,6 @@ __device__ __forceinline__ void coarse_apply(const CoarseArgs &a, long long me, 
             H3D_LB(25) H3D_LB(26)
 #undef H3D_LB
         }
-        const int Kn = K ^ ((dx & 1) | ((dy & 1) << 1) | ((dz & 1) << 2));
         const unsigned nid = (unsigned)Kn * (unsigned)a.P + X[dx + 1] + Y[dy + 1] + Z[dz + 1];
         const float *up = a.u + fidx(3 * cb, nid);  // planes 3cb.. of the neighbour, FVB apart
 #pragma unroll
@@ -141,11 +143,15 @@ __device__ __forceinline__ void coarse_task(long long &p, int &cb, unsigned bid)
     p = (long long)(bid / NG) * blockDim.x + threadIdx.x;
 }
 
-// RES (the last colour of a sweep, whose neighbours are final) also writes the
-// residual of the updated vertex: r = f - acc - A_0 u with acc the neighbour sum.
+// ZERO: the sweep of a V-cycle's down leg, which starts from u = 0.  u is not read
+// before it is written (nor cleared), a colour sees only the neighbours of the earlier
+// ones (the others are still 0: the same sums), and the vertex's residual so far, r = f
+// - acc - A_0 u, is written; the residual launch takes the later colours' share from it
+// (k_coarse_residual), so the two together read each stencil about once instead of
+// twice.
 // bid: the CTA's index in the design's launch (blockIdx.x, or its slice of a
 // batched launch)
-template <int K, bool F32, int CGS_CPT, bool RES>
+template <int K, bool F32, int CGS_CPT, bool ZERO>
 __device__ __forceinline__ void coarse_gs_block(const CoarseArgs &a, unsigned bid) {
     long long p;
     int cb;
@@ -155,21 +161,21 @@ __device__ __forceinline__ void coarse_gs_block(const CoarseArgs &a, unsigned bi
     int i, j, l;
     cplane_coords(a, p, i, j, l);
     float acc[3 * CGS_CPT], ks[9];
-    coarse_apply<K, false, F32, CGS_CPT>(a, me, i, j, l, cb, acc);
+    coarse_apply<K, false, F32, CGS_CPT, false, ZERO ? -1 : 0>(a, me, i, j, l, cb, acc);
     load_block<13, F32>(a, me, ks);
     const float w = a.w;
 #pragma unroll
     for (int c = 0; c < CGS_CPT; ++c) {
         float *u = a.u + fidx(3 * (cb + c), me);
         const float *f = a.f + fidx(3 * (cb + c), me);
-        float u0 = u[0], u1 = u[FVB], u2 = u[2 * FVB];
+        float u0 = ZERO ? 0.f : u[0], u1 = ZERO ? 0.f : u[FVB], u2 = ZERO ? 0.f : u[2 * FVB];
         u0 = w * (f[0] - acc[3 * c] - ks[1] * u1 - ks[2] * u2) / ks[0] + (1.f - w) * u0;
         u1 = w * (f[FVB] - acc[3 * c + 1] - ks[3] * u0 - ks[5] * u2) / ks[4] + (1.f - w) * u1;
         u2 = w * (f[2 * FVB] - acc[3 * c + 2] - ks[6] * u0 - ks[7] * u1) / ks[8] + (1.f - w) * u2;
         u[0] = u0;
         u[FVB] = u1;
         u[2 * FVB] = u2;
-        if (RES) {
+        if (ZERO) {
             float *r = a.r + fidx(3 * (cb + c), me);
 #pragma unroll
             for (int m = 0; m < 3; ++m)
@@ -178,27 +184,29 @@ __device__ __forceinline__ void coarse_gs_block(const CoarseArgs &a, unsigned bi
     }
 }
 
-template <int K, bool F32, int CGS_CPT, int CGS_MINB, bool RES = false>
+template <int K, bool F32, int CGS_CPT, int CGS_MINB, bool ZERO = false>
 __global__ void __launch_bounds__(128, CGS_MINB) k_coarse_gs(CoarseArgs a) {
-    coarse_gs_block<K, F32, CGS_CPT, RES>(a, blockIdx.x);
+    coarse_gs_block<K, F32, CGS_CPT, ZERO>(a, blockIdx.x);
 }
 
-template <bool F32, int CRES_CPT>
+// AFTER: the residual after a ZERO sweep, r -= sum of A_d u over the neighbours of later
+// colours (their whole change since r was written)
+template <bool F32, int CRES_CPT, bool AFTER>
 __device__ __forceinline__ void coarse_res_vertex(const CoarseArgs &a, long long p, int cb, int K) {
     const long long me = (long long)K * a.P + p;
     int i, j, l;
     cplane_coords(a, p, i, j, l);
     float acc[3 * CRES_CPT];
-    coarse_apply<-1, true, F32, CRES_CPT>(a, me, i, j, l, cb, acc, K);
+    coarse_apply<-1, !AFTER, F32, CRES_CPT, false, AFTER ? 1 : 0>(a, me, i, j, l, cb, acc, K);
 #pragma unroll
     for (int q = 0; q < 3 * CRES_CPT; ++q) {
         const long long o = fidx(3 * cb + q, me);
-        a.r[o] = a.f[o] - acc[q];
+        a.r[o] = (AFTER ? a.r[o] : a.f[o]) - acc[q];
     }
 }
 
-// all colours in one launch (eight, or seven after a sweep whose last colour wrote
-// its own residual), the colour the block index modulo NCOL and a run-time value
+// all colours in one launch (eight, or seven after a ZERO sweep, whose last colour's r
+// is final), the colour the block index modulo NCOL and a run-time value
 // of one code body: the CTAs of one vertex block read each other's neighbour rows
 // while they are in L2, and a small level costs one launch instead of eight
 template <bool F32, int CRES_CPT, unsigned NCOL>
@@ -209,7 +217,7 @@ __device__ __forceinline__ void coarse_residual_block(const CoarseArgs &a, unsig
     const int cb = (int)(bx % NG) * CRES_CPT;
     const long long p = (long long)(bx / NG) * blockDim.x + threadIdx.x;
     if (p >= a.P) return;
-    coarse_res_vertex<F32, CRES_CPT>(a, p, cb, K);
+    coarse_res_vertex<F32, CRES_CPT, NCOL == 7>(a, p, cb, K);
 }
 
 template <bool F32, int CRES_CPT, int CRES_MINB, unsigned NCOL>
@@ -292,22 +300,24 @@ static void coarse_residual_shape(const Level &L, const CoarseArgs &a, cudaStrea
 
 void launch_coarse_residual(const Level &L, cudaStream_t s) { coarse_residual_shape<8>(L, make_cargs(L), s); }
 
-// a sweep followed by the level's residual: the last colour's launch writes its
-// own residual, the residual launch covers the other seven colours
+// the down leg of a level: the sweep from u = 0, each colour's launch writing its
+// residual so far, then the later colours' share of the residual of all but the last.
+// Level 1 of a 256^3 grid (128^3, FP16 stencils): the residual 255 -> 128 us; all levels'
+// down legs of a 256^3 solve (10 cycles) together 4.9 ms less.
 template <bool F32, int C, int MINB>
 static void coarse_gs_sweep_res(const CoarseArgs &a, cudaStream_t s) {
     const unsigned nb = (unsigned)((a.P + 127) / 128) * (NCASE / C);
-    k_coarse_gs<0, F32, C, MINB><<<nb, 128, 0, s>>>(a);
-    k_coarse_gs<1, F32, C, MINB><<<nb, 128, 0, s>>>(a);
-    k_coarse_gs<2, F32, C, MINB><<<nb, 128, 0, s>>>(a);
-    k_coarse_gs<3, F32, C, MINB><<<nb, 128, 0, s>>>(a);
-    k_coarse_gs<4, F32, C, MINB><<<nb, 128, 0, s>>>(a);
-    k_coarse_gs<5, F32, C, MINB><<<nb, 128, 0, s>>>(a);
-    k_coarse_gs<6, F32, C, MINB><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<0, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<1, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<2, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<3, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<4, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<5, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
+    k_coarse_gs<6, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
     k_coarse_gs<7, F32, C, MINB, true><<<nb, 128, 0, s>>>(a);
 }
 
-void launch_coarse_gs_residual(const Level &L, float w, cudaStream_t s) {
+void launch_coarse_down(const Level &L, float w, cudaStream_t s) {
     CoarseArgs a = make_cargs(L);
     a.w = w;
     if (L.st32) {
@@ -395,10 +405,10 @@ __global__ void __launch_bounds__(256) k_prolong(Planes F, Planes C, int r0, int
 // of each colour plane.  Fine vertex 2X + o has the colour of o's parities and, in
 // that colour's plane, the coordinates X - [o < 0] (wrapped) per axis; the sums
 // run in the general kernel's order, so the results are identical.
-// thread t of case c; uc (or nullptr): the coarse solution, cleared at the vertex
+// thread t of case c
 __device__ __forceinline__ void restrict2_thread(const Planes &F, const Planes &C, const FastDiv &dn0,
                                                  const FastDiv &dn1, const float *__restrict__ rf, float *fc,
-                                                 float *uc, long long t, int c) {
+                                                 long long t, int c) {
     if (t >= C.nv) return;
     const unsigned q = (unsigned)t, tq = dn0.div(q), zq = dn1.div(tq);
     const int x = (int)(q - tq * (unsigned)C.n[0]), y = (int)(tq - zq * (unsigned)C.n[1]), z = (int)zq;
@@ -425,17 +435,11 @@ __device__ __forceinline__ void restrict2_thread(const Planes &F, const Planes &
     dst[0] = a0;
     dst[FVB] = a1;
     dst[2 * FVB] = a2;
-    if (uc) {
-        float *z0 = uc + fidx(3 * c, cv);
-        z0[0] = 0.f;
-        z0[FVB] = 0.f;
-        z0[2 * FVB] = 0.f;
-    }
 }
 
 __global__ void __launch_bounds__(256) k_restrict2(Planes F, Planes C, FastDiv dn0, FastDiv dn1,
                                                    const float *__restrict__ rf, float *fc) {
-    restrict2_thread(F, C, dn0, dn1, rf, fc, nullptr, blockIdx.x * (long long)blockDim.x + threadIdx.x, blockIdx.y);
+    restrict2_thread(F, C, dn0, dn1, rf, fc, blockIdx.x * (long long)blockDim.x + threadIdx.x, blockIdx.y);
 }
 
 // Ratio 2: one thread per coarse cell X; its eight fine vertices 2X + e take
@@ -680,9 +684,8 @@ void launch_stencil_from_lex(const Level &L, const float *src_lex, cudaStream_t 
 // whatever the level's size).  k_vcycle_bottom runs the V-cycle's steps from the
 // restriction into level `first` down to the coarsest solve and back up to the
 // post-smoothing of level `first` as phases of one cooperative launch, separated by
-// grid-wide barriers: per smoothed level on the way down, restriction (and the
-// cleared correction), eight colours (the last with its residual), the residual of
-// the other seven colours; at the bottom the restriction and the dense coarsest
+// grid-wide barriers: per smoothed level on the way down, restriction, eight colours
+// from a zero correction, the later colours' share of the residual; at the bottom the restriction and the dense coarsest
 // solve; per level on the way up, prolongation and eight colours.  Each phase runs
 // the arithmetic of the separate kernels in the same order (two load cases per
 // thread, ratio-2 transfers), so the results are the same to the last bit.  Values
@@ -733,7 +736,7 @@ __device__ __forceinline__ bool bottom_sync(unsigned *bar, int *flag) {
     return gone == 0;
 }
 
-// restriction (ratio 2) of F's residual into C's right-hand side, C's correction cleared
+// restriction (ratio 2) of F's residual into C's right-hand side
 __device__ void bottom_restrict(const CoarseArgs &Fa, const Planes &F, const CoarseArgs &Ca, const Planes &C) {
     const long long total = C.nv * NCASE;
     for (long long t = blockIdx.x * (long long)BOT_T + threadIdx.x; t < total; t += (long long)gridDim.x * BOT_T) {
@@ -763,9 +766,6 @@ __device__ void bottom_restrict(const CoarseArgs &Fa, const Planes &F, const Coa
         dst[FVB] = a1;
         dst[2 * FVB] = a2;
     }
-    const long long nu = field_floats(C.nv);
-    for (long long t = blockIdx.x * (long long)BOT_T + threadIdx.x; t < nu; t += (long long)gridDim.x * BOT_T)
-        Ca.u[t] = 0.f;
 }
 
 // trilinear prolongation (ratio 2) of C's correction into F's
@@ -807,11 +807,10 @@ __device__ void bottom_prolong(const CoarseArgs &Fa, const Planes &F, const Coar
     }
 }
 
-// one colour K of the sweep (two load cases per thread); RES: also the residual
-template <bool F32, int K, bool RES>
+// one colour K of the sweep (two load cases per thread); ZERO: as in coarse_gs_block
+template <bool F32, int K, bool ZERO>
 __device__ void bottom_gs_k(const CoarseArgs &a) {
     constexpr int C = 2, NG = NCASE / C;
-    constexpr bool res = RES;
     const long long nvb = (a.P + BOT_T - 1) / BOT_T * NG;
     for (long long b = blockIdx.x; b < nvb; b += gridDim.x) {
         const int cb = (int)(b % NG) * C;
@@ -821,7 +820,7 @@ __device__ void bottom_gs_k(const CoarseArgs &a) {
         int i, j, l;
         cplane_coords(a, p, i, j, l);
         float acc[3 * C], ks[9];
-        coarse_apply<K, false, F32, C, true>(a, me, i, j, l, cb, acc);
+        coarse_apply<K, false, F32, C, true, ZERO ? -1 : 0>(a, me, i, j, l, cb, acc);
         load_block<13, F32>(a, me, ks);
         const float w = a.w;
 #pragma unroll
@@ -829,14 +828,14 @@ __device__ void bottom_gs_k(const CoarseArgs &a) {
             float *u = a.u + fidx(3 * (cb + c), me);
             const float *f = a.f + fidx(3 * (cb + c), me);
             const float f0 = __ldcg(f), f1 = __ldcg(f + FVB), f2 = __ldcg(f + 2 * FVB);
-            float u0 = __ldcg(u), u1 = __ldcg(u + FVB), u2 = __ldcg(u + 2 * FVB);
+            float u0 = ZERO ? 0.f : __ldcg(u), u1 = ZERO ? 0.f : __ldcg(u + FVB), u2 = ZERO ? 0.f : __ldcg(u + 2 * FVB);
             u0 = w * (f0 - acc[3 * c] - ks[1] * u1 - ks[2] * u2) / ks[0] + (1.f - w) * u0;
             u1 = w * (f1 - acc[3 * c + 1] - ks[3] * u0 - ks[5] * u2) / ks[4] + (1.f - w) * u1;
             u2 = w * (f2 - acc[3 * c + 2] - ks[6] * u0 - ks[7] * u1) / ks[8] + (1.f - w) * u2;
             u[0] = u0;
             u[FVB] = u1;
             u[2 * FVB] = u2;
-            if (res) {
+            if (ZERO) {
                 float *r = a.r + fidx(3 * (cb + c), me);
                 const float ff[3] = {f0, f1, f2};
 #pragma unroll
@@ -847,24 +846,21 @@ __device__ void bottom_gs_k(const CoarseArgs &a) {
     }
 }
 
-template <bool F32>
-__device__ void bottom_gs(const CoarseArgs &a, int K, bool res) {
+template <bool F32, bool ZERO>
+__device__ void bottom_gs(const CoarseArgs &a, int K) {
     switch (K) {
-    case 0: bottom_gs_k<F32, 0, false>(a); break;
-    case 1: bottom_gs_k<F32, 1, false>(a); break;
-    case 2: bottom_gs_k<F32, 2, false>(a); break;
-    case 3: bottom_gs_k<F32, 3, false>(a); break;
-    case 4: bottom_gs_k<F32, 4, false>(a); break;
-    case 5: bottom_gs_k<F32, 5, false>(a); break;
-    case 6: bottom_gs_k<F32, 6, false>(a); break;
-    default:
-        if (res) bottom_gs_k<F32, 7, true>(a);
-        else bottom_gs_k<F32, 7, false>(a);
-        break;
+    case 0: bottom_gs_k<F32, 0, ZERO>(a); break;
+    case 1: bottom_gs_k<F32, 1, ZERO>(a); break;
+    case 2: bottom_gs_k<F32, 2, ZERO>(a); break;
+    case 3: bottom_gs_k<F32, 3, ZERO>(a); break;
+    case 4: bottom_gs_k<F32, 4, ZERO>(a); break;
+    case 5: bottom_gs_k<F32, 5, ZERO>(a); break;
+    case 6: bottom_gs_k<F32, 6, ZERO>(a); break;
+    default: bottom_gs_k<F32, 7, ZERO>(a); break;
     }
 }
 
-// the residual of colours 0..6 (colour 7's came with its sweep)
+// the later colours' share of the residual of colours 0..6 (colour 7's is final)
 template <bool F32>
 __device__ void bottom_residual(const CoarseArgs &a) {
     constexpr int C = 2, NG = NCASE / C, NCOL = 7;
@@ -879,11 +875,11 @@ __device__ void bottom_residual(const CoarseArgs &a) {
         int i, j, l;
         cplane_coords(a, p, i, j, l);
         float acc[3 * C];
-        coarse_apply<-1, true, F32, C, true>(a, me, i, j, l, cb, acc, K);
+        coarse_apply<-1, false, F32, C, true, 1>(a, me, i, j, l, cb, acc, K);
 #pragma unroll
         for (int q = 0; q < 3 * C; ++q) {
             const long long o = fidx(3 * cb + q, me);
-            a.r[o] = __ldcg(a.f + o) - acc[q];
+            a.r[o] = __ldcg(a.r + o) - acc[q];
         }
     }
 }
@@ -902,7 +898,7 @@ __global__ void __launch_bounds__(BOT_T) k_vcycle_bottom(const __grid_constant__
         bottom_restrict(A.lv[l - 1], A.P[l - 1], A.lv[l], A.P[l]);
         if (!bottom_sync(A.bar, A.flag)) return;
         for (int K = 0; K < 8; ++K) {
-            bottom_gs<F32>(A.lv[l], K, K == 7);
+            bottom_gs<F32, true>(A.lv[l], K);
             if (!bottom_sync(A.bar, A.flag)) return;
         }
         bottom_residual<F32>(A.lv[l]);
@@ -916,7 +912,7 @@ __global__ void __launch_bounds__(BOT_T) k_vcycle_bottom(const __grid_constant__
         bottom_prolong(A.lv[l], A.P[l], A.lv[l + 1], A.P[l + 1]);
         if (!bottom_sync(A.bar, A.flag)) return;
         for (int K = 0; K < 8; ++K) {
-            bottom_gs<F32>(A.lv[l], K, false);
+            bottom_gs<F32, false>(A.lv[l], K);
             if (l > 1 || K < 7)
                 if (!bottom_sync(A.bar, A.flag)) return;
         }
@@ -999,7 +995,7 @@ struct CoarseBatchTab {
 
 // C cases per thread at MB CTAs per SM: launch shape 0 (C = 2, 6 CTAs/SM) or 1
 // (C = 6, 4 CTAs/SM)
-template <int K, bool F32, bool RES, int C, int MB>
+template <int K, bool F32, bool ZERO, int C, int MB>
 __global__ void __launch_bounds__(128, MB) k_coarse_gs_batch(const CoarseBatchTab *__restrict__ t,
                                                            const int *__restrict__ active) {
     __shared__ __align__(16) unsigned buf[sizeof(CoarseArgs) / 4];
@@ -1008,7 +1004,7 @@ __global__ void __launch_bounds__(128, MB) k_coarse_gs_batch(const CoarseBatchTa
     const CoarseEnt &en = t->e[i];
     if (!__ldg(&active[en.design])) return;
     const CoarseArgs &a = stage_args(en.a, buf);
-    coarse_gs_block<K, F32, C, RES>(a, blockIdx.x - __ldg(&sl.start[i]));
+    coarse_gs_block<K, F32, C, ZERO>(a, blockIdx.x - __ldg(&sl.start[i]));
 }
 
 template <bool F32>
@@ -1059,33 +1055,35 @@ int coarse_batch_create(const Level *const *lv, const int *design, int n, bool s
     return rc;
 }
 
-template <bool F32, int C, int MB>
-static void coarse_sweep_batch(const BatchTab &t, const int *active, bool residual, cudaStream_t s) {
+template <bool F32, int C, int MB, bool ZERO>
+static void coarse_sweep_batch(const BatchTab &t, const int *active, cudaStream_t s) {
     const CoarseBatchTab *d = static_cast<const CoarseBatchTab *>(t.dev);
     const unsigned g = C == BATCH_CPT ? t.grid[0] : t.grid[2];
-    k_coarse_gs_batch<0, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    k_coarse_gs_batch<1, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    k_coarse_gs_batch<2, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    k_coarse_gs_batch<3, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    k_coarse_gs_batch<4, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    k_coarse_gs_batch<5, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    k_coarse_gs_batch<6, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    if (residual) {
-        k_coarse_gs_batch<7, F32, true, C, MB><<<g, 128, 0, s>>>(d, active);
-        k_coarse_residual_batch<F32><<<t.grid[1], 128, 0, s>>>(d, active);
-    } else {
-        k_coarse_gs_batch<7, F32, false, C, MB><<<g, 128, 0, s>>>(d, active);
-    }
+    k_coarse_gs_batch<0, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<1, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<2, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<3, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<4, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<5, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<6, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    k_coarse_gs_batch<7, F32, ZERO, C, MB><<<g, 128, 0, s>>>(d, active);
+    if (ZERO) k_coarse_residual_batch<F32><<<t.grid[1], 128, 0, s>>>(d, active);
 }
 
-void launch_coarse_sweep_batch(const BatchTab &t, bool f32, const int *active, bool residual, int shape,
+template <bool F32, int C, int MB>
+static void coarse_sweep_batch(const BatchTab &t, const int *active, bool down, cudaStream_t s) {
+    if (down) coarse_sweep_batch<F32, C, MB, true>(t, active, s);
+    else coarse_sweep_batch<F32, C, MB, false>(t, active, s);
+}
+
+void launch_coarse_sweep_batch(const BatchTab &t, bool f32, const int *active, bool down, int shape,
                                cudaStream_t s) {
     if (f32) {
-        if (shape == 1) coarse_sweep_batch<true, 6, 4>(t, active, residual, s);
-        else coarse_sweep_batch<true, BATCH_CPT, BATCH_MINB>(t, active, residual, s);
+        if (shape == 1) coarse_sweep_batch<true, 6, 4>(t, active, down, s);
+        else coarse_sweep_batch<true, BATCH_CPT, BATCH_MINB>(t, active, down, s);
     } else {
-        if (shape == 1) coarse_sweep_batch<false, 6, 4>(t, active, residual, s);
-        else coarse_sweep_batch<false, BATCH_CPT, BATCH_MINB>(t, active, residual, s);
+        if (shape == 1) coarse_sweep_batch<false, 6, 4>(t, active, down, s);
+        else coarse_sweep_batch<false, BATCH_CPT, BATCH_MINB>(t, active, down, s);
     }
 }
 
@@ -1111,7 +1109,7 @@ __global__ void __launch_bounds__(256) k_restrict_batch(const TransferBatchTab *
     if (!__ldg(&active[t->e[i].design])) return;
     const TransferEnt &e = stage_args(t->e[i], buf);
     const long long tt = (long long)(blockIdx.x - __ldg(&t->sl.start[i])) * blockDim.x + threadIdx.x;
-    restrict2_thread(e.F, e.C, e.dn0, e.dn1, e.rf, e.fc, e.uc, tt, blockIdx.y);
+    restrict2_thread(e.F, e.C, e.dn0, e.dn1, e.rf, e.fc, tt, blockIdx.y);
 }
 
 __global__ void __launch_bounds__(256) k_prolong_batch(const TransferBatchTab *__restrict__ t,
