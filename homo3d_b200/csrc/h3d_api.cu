@@ -750,7 +750,7 @@ int elastic_prepare(h3d_handle *h) {
 }
 
 // store the solutions as chi and enqueue the energy reduction of the 21 entries
-// of C, with the results and the kernel's wait flag copied to the host
+// of C, with the results copied to the host
 int elastic_enqueue_energy(h3d_handle *h) {
     Level &L = h->lv[0];
     cudaStream_t s = h->stream;
@@ -758,23 +758,16 @@ int elastic_enqueue_energy(h3d_handle *h) {
         CK(cudaMemcpyAsync(h->chi, h->u64, sizeof(double) * field_floats(L.P.nv), cudaMemcpyDeviceToDevice, s));
     else launch_convert_field(L.P.nv, L.u, h->chi, s);
     h->chi_zero = false;
-    int nsm = 0;
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-    const int eb = energy_tc_blocks(L.P, nsm);
-    CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), s));
-    if (launch_elastic_tc(L.P, h->chi, h->rho, h->ke, h->partial, eb, h->d_flag, s) != 0)
-        return fail(h, H3D_ERR_CUDA, "tensor-core energy kernel could not be configured");
+    const int eb = energy_blocks(L.P, h->num_sms);
+    launch_elastic(L.P, h->chi, h->rho, h->ked, h->partial, eb, s);
     launch_elastic_finish(h->partial, eb, h->d_small, s);
     CKL();
     CK(cudaMemcpyAsync(h->h_small, h->d_small, sizeof(double) * 21, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&h->h_small[63], h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     return H3D_OK;
 }
 
 // C from the reduced energies once the stream has drained
 int elastic_read(h3d_handle *h, double *C) {
-    if (*reinterpret_cast<int *>(&h->h_small[63]))
-        return fail(h, H3D_ERR_CUDA, "tensor-core energy kernel: mbarrier wait timed out");
     const double vol = (double)h->lv[0].P.nv;
     int t = 0;
     for (int i = 0; i < 6; i++)
@@ -1846,18 +1839,11 @@ int h3d_sensitivity(h3d_handle *h, const float dC[36], float *sens_dev, int pitc
     const Planes &P = h->lv[0].P;
     if (pitchT < 0) pitchT = P.n[0];
     if (pitchT < P.n[0]) return fail(h, H3D_ERR_ARG, "pitchT smaller than the x resolution");
-    CK(cudaMemsetAsync(sens_dev, 0, sizeof(float) * (size_t)pitchT * P.n[1] * P.n[2], h->stream));
-    int nsm = 0;
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-    CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->stream));
-    if (launch_sensitivity_tc(P, h->chi, h->ke, dC, sens_dev, pitchT, energy_tc_blocks(P, nsm), h->d_flag,
-                              h->stream) != 0)
-        return fail(h, H3D_ERR_CUDA, "tensor-core energy kernel could not be configured");
+    if (pitchT != P.n[0])  // the padding
+        CK(cudaMemsetAsync(sens_dev, 0, sizeof(float) * (size_t)pitchT * P.n[1] * P.n[2], h->stream));
+    launch_sensitivity(P, h->chi, h->ked, dC, sens_dev, pitchT, h->stream);
     CKL();
-    CK(cudaMemcpyAsync(&h->h_small[63], h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    if (*reinterpret_cast<int *>(&h->h_small[63]))
-        return fail(h, H3D_ERR_CUDA, "tensor-core energy kernel: mbarrier wait timed out");
     return H3D_OK;
 }
 
@@ -1992,16 +1978,11 @@ int h3d_design_step(h3d_handle *h, const float dC[36], float *rho_dev, float *se
         h->dgraph = nullptr;
     }
     if (!h->dgraph) {
-        if (configure_energy_tc() != 0) return fail(h, H3D_ERR_CUDA, "tensor-core energy kernel could not be configured");
-        int nsm = 0;
-        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
         cudaStream_t s = h->stream;
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         cudaMemcpyAsync(h->d_dcw, h->h_dcw, sizeof(float) * 21, cudaMemcpyHostToDevice, s);
-        cudaMemsetAsync(h->d_flag, 0, sizeof(int), s);
-        cudaMemsetAsync(sens_dev, 0, sizeof(float) * ne, s);
-        launch_sensitivity_tc_dev(P, h->chi, h->ke, h->d_dcw, sens_dev, n[0], energy_tc_blocks(P, nsm), h->d_flag, s);
+        launch_sensitivity_dev(P, h->chi, h->ked, h->d_dcw, sens_dev, n[0], s);
         launch_penalize(ne, rho_dev, sens_dev, prm->penal, 1, s);
         if (prm->sym >= 0) launch_symmetrize(n, sens_dev, prm->sym, s);
         if (prm->filter_radius > 0) {
@@ -2012,7 +1993,6 @@ int h3d_design_step(h3d_handle *h, const float dC[36], float *rho_dev, float *se
         launch_oc(sens_dev, rho_dev, h->tmp, ne, prm->volratio, prm->min_rho, prm->step_limit, prm->damp, h->partial,
                   s);
         if (prm->sym >= 0) launch_symmetrize(n, rho_dev, prm->sym, s);
-        cudaMemcpyAsync(&h->h_small[63], h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s);
         CK(cudaStreamEndCapture(s, &g));
         cudaError_t e = cudaGraphInstantiate(&h->dgraph, g, 0);
         cudaGraphDestroy(g);
@@ -2027,8 +2007,6 @@ int h3d_design_step(h3d_handle *h, const float dC[36], float *rho_dev, float *se
     sensitivity_weights(P, dC, h->h_dcw);
     CK(cudaGraphLaunch(h->dgraph, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    if (*reinterpret_cast<int *>(&h->h_small[63]))
-        return fail(h, H3D_ERR_CUDA, "tensor-core energy kernel: mbarrier wait timed out");
     return H3D_OK;
 }
 

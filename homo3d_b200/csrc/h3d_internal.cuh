@@ -366,22 +366,18 @@ int configure_fine_residual_tc();
 int fine_residual_tc_blocks(const Planes &P, int num_sms);
 int launch_fine_residual_tc(const Level &L, const float *rho, const KeMat &ke, double *partial, int nblk,
                             int *flag, cudaStream_t s);
-// homogenized tensor and sensitivities on the tensor cores (k_homog_tc.cu):
-// a persistent grid of energy_tc_blocks CTAs; *flag is set if an mbarrier wait
-// timed out; the launchers return -1 when the kernel cannot be configured
-int energy_tc_blocks(const Planes &P, int num_sms);
-int launch_elastic_tc(const Planes &P, const double *chi, const float *rho, const KeMat &ke, double *partial,
-                      int nblk, int *flag, cudaStream_t s);
-int launch_sensitivity_tc(const Planes &P, const double *chi, const KeMat &ke, const float *dc36, float *sens,
-                          int pitch, int nblk, int *flag, cudaStream_t s);
+// homogenized tensor and sensitivities (k_homog.cu); ked: the FP64 element matrix
+int energy_blocks(const Planes &P, int num_sms);
+void launch_elastic(const Planes &P, const double *chi, const float *rho, const double *ked, double *partial, int nblk,
+                    cudaStream_t s);
+void launch_sensitivity(const Planes &P, const double *chi, const double *ked, const float *dc36, float *sens, int pitch,
+                        cudaStream_t s);
 void launch_elastic_finish(const double *partial, int nblk, double *out21, cudaStream_t s);
 // the same sensitivity with its 21 weights (sensitivity_weights) read from device
-// memory at run time, for captured graphs; configure_energy_tc first (outside any
-// capture), -1 if the kernels cannot be configured
+// memory at run time, for captured graphs
 void sensitivity_weights(const Planes &P, const float *dc36, float w21[21]);
-int configure_energy_tc();
-void launch_sensitivity_tc_dev(const Planes &P, const double *chi, const KeMat &ke, const float *dcw, float *sens,
-                               int pitch, int nblk, int *flag, cudaStream_t s);
+void launch_sensitivity_dev(const Planes &P, const double *chi, const double *ked, const float *dcw, float *sens,
+                            int pitch, cudaStream_t s);
 // design (k_design.cu)
 void launch_density_in(const int n[3], const float *src, int pitch, float *dst, cudaStream_t s);
 void launch_penalize(long long n, const float *rho, float *out, float p, int backward, cudaStream_t s);
