@@ -167,8 +167,9 @@ struct h3d_handle {
     cudaGraphExec_t vgraph = nullptr;   // one V-cycle on the level-0 field u
     cudaGraphExec_t rgraph = nullptr;   // refinement step: u64 += u, f = f0 - K u64 (FP32 products)
     cudaGraphExec_t xgraph = nullptr;   // the same with the FP64-accumulated residual
-    cudaGraphExec_t sgraph = nullptr;   // a solve's V-cycle: vgraph + rigid-translation deflation
-    cudaGraphExec_t fgraph = nullptr;   // coarsest assembly + Gauss-Jordan inverse (one launch per panel)
+    // [1]: with the stencils of the FP32 fallback (wide)
+    cudaGraphExec_t sgraph[2] = {};     // a solve's V-cycle: vgraph + rigid-translation deflation
+    cudaGraphExec_t fgraph[2] = {};     // coarsest assembly + Gauss-Jordan inverse (one launch per panel)
     cudaGraphExec_t dgraph = nullptr;   // design step (h3d_design_step)
     float *d_dcw = nullptr, *h_dcw = nullptr;  // sensitivity weights: device copy, pinned host source
     h3d_design_params dkey{};           // parameters and buffers the design graph was captured for
@@ -188,6 +189,13 @@ struct h3d_handle {
     unsigned *d_bar = nullptr;          // its grid-barrier state
     int *d_botflag = nullptr;           // set if one of its barrier waits ran out
     bool have_density = false, have_stencils = false;
+    // FP32 fallback of an FP16 hierarchy (SolveRun::widen).  wide: lv[].st and aug are
+    // the FP32 ones, from the cycle a solve needs them to its end; st_alt, aug_alt: the
+    // ones not in use (null until the first fallback)
+    bool wide = false;
+    uint4 *st_alt[MAXLV] = {};
+    double *aug_alt = nullptr;
+    unsigned custom = 0;  // levels whose stencils come from h3d_set_field, not from the density
     bool tuned = false;  // launch shapes chosen (autotuner or h3d_set_tuning)
     // chi_zero: the stored solutions chi are all zero (allocation, h3d_reset_solutions,
     // no write since); u64_zero: the FP64 solution was set to zero by the last
@@ -265,10 +273,12 @@ void build_q(const double ke[576], const int r[3], std::vector<float> &q, int &n
 
 int destroy_graph(h3d_handle *h) {
     if (h->vgraph) { cudaGraphExecDestroy(h->vgraph); h->vgraph = nullptr; }
+    for (int w = 0; w < 2; w++) {
+        if (h->sgraph[w]) { cudaGraphExecDestroy(h->sgraph[w]); h->sgraph[w] = nullptr; }
+        if (h->fgraph[w]) { cudaGraphExecDestroy(h->fgraph[w]); h->fgraph[w] = nullptr; }
+    }
     if (h->rgraph) { cudaGraphExecDestroy(h->rgraph); h->rgraph = nullptr; }
     if (h->xgraph) { cudaGraphExecDestroy(h->xgraph); h->xgraph = nullptr; }
-    if (h->sgraph) { cudaGraphExecDestroy(h->sgraph); h->sgraph = nullptr; }
-    if (h->fgraph) { cudaGraphExecDestroy(h->fgraph); h->fgraph = nullptr; }
     if (h->dgraph) { cudaGraphExecDestroy(h->dgraph); h->dgraph = nullptr; }
     return H3D_OK;
 }
@@ -379,7 +389,7 @@ int enqueue_zero_start(h3d_handle *h) {
 // rgraph / xgraph: the refinement step with FP32 / FP64 accumulation of the residual
 enum GraphKind { G_VCYCLE, G_SOLVE, G_REFINE, G_REFINE_EXACT };
 int build_graph(h3d_handle *h, GraphKind kind) {
-    cudaGraphExec_t &ge = kind == G_VCYCLE ? h->vgraph : kind == G_SOLVE ? h->sgraph
+    cudaGraphExec_t &ge = kind == G_VCYCLE ? h->vgraph : kind == G_SOLVE ? h->sgraph[h->wide]
                         : kind == G_REFINE_EXACT ? h->xgraph : h->rgraph;
     if (ge) return H3D_OK;
     cudaGraph_t g = nullptr;
@@ -463,6 +473,109 @@ int autotune(h3d_handle *h) {
 
 namespace {
 
+// the coarsest level's assembly and Gauss-Jordan inversion with the
+// singular-matrix flag copied to the host; factor_coarsest_check reads it once
+// the stream has drained
+int factor_coarsest_enqueue(h3d_handle *h) {
+    cudaStream_t s = h->stream;
+    cudaGraphExec_t &ge = h->fgraph[h->wide];
+    if (!ge) {
+        cudaGraph_t g = nullptr;
+        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        launch_coarse_assemble(h->lv[h->nl - 1], h->aug, s);
+        cudaMemsetAsync(h->d_flag, 0, sizeof(int), s);
+        launch_gauss_jordan(h->aug, h->ndof, h->d_flag, s);
+        CK(cudaStreamEndCapture(s, &g));
+        cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            ge = nullptr;
+            return fail(h, H3D_ERR_CUDA, std::string("graph: ") + cudaGetErrorString(e));
+        }
+    }
+    CK(cudaGraphLaunch(ge, s));
+    CK(cudaMemcpyAsync(&h->h_small[63], h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    return H3D_OK;
+}
+
+int factor_coarsest_check(h3d_handle *h) {
+    int flag = 0;
+    std::memcpy(&flag, &h->h_small[63], sizeof(int));
+    if (flag) return fail(h, H3D_ERR_SINGULAR, "coarsest-grid matrix is singular");
+    h->have_stencils = true;
+    return H3D_OK;
+}
+
+// level l's stencils from the next finer level's (level 1: from the densities)
+void enqueue_stencil(h3d_handle *h, int l) {
+    if (l == 1) {
+        launch_galerkin_l1(h->lv[0], h->lv[1], h->rho, h->q, h->nsub, h->stream);
+        launch_dirichlet_patch(h->lv[0], h->lv[1], h->rho, h->d_ked, h->cfg.pin_mode == H3D_PIN_IDENTITY, h->stream);
+    } else {
+        launch_galerkin(h->lv[l - 1], h->lv[l], h->stream);
+    }
+}
+
+// the coarse levels onto the FP32 fallback's stencils and coarsest inverse, or back
+void use_wide(h3d_handle *h, bool on) {
+    if (h->wide == on) return;
+    for (int l = 1; l < h->nl; l++) {
+        std::swap(h->lv[l].st, h->st_alt[l]);
+        h->lv[l].st32 = on;
+    }
+    std::swap(h->aug, h->aug_alt);
+    h->wide = on;
+}
+
+// whether a solve can fall back to FP32 stencils: FP16 ones, all built from the density
+bool can_widen(const h3d_handle *h) { return !h->wide && !h->lv[1].st32 && h->have_density && !h->custom; }
+
+// The coarse levels with FP32 stencils, beside the FP16 ones; false if there is no
+// memory or the coarsest matrix is singular, and the FP16 ones stay in use then.
+bool widen_stencils(h3d_handle *h, int &err) {
+    err = H3D_OK;
+    bool fits = true;
+    for (int l = 1; l < h->nl && fits; l++) {
+        if (h->st_alt[l]) continue;
+        const size_t sb = sizeof(uint4) * NCHUNK32 * (size_t)h->lv[l].P.nv;
+        fits = cudaMalloc(&h->st_alt[l], sb) == cudaSuccess &&
+               cudaMemsetAsync(h->st_alt[l], 0, sb, h->stream) == cudaSuccess;
+    }
+    if (fits && !h->aug_alt)
+        fits = cudaMalloc(&h->aug_alt, sizeof(double) * gauss_jordan_doubles(h->ndof)) == cudaSuccess;
+    if (!fits) {
+        cudaGetLastError();
+        for (int l = 1; l < h->nl; l++) {
+            cudaFree(h->st_alt[l]);
+            h->st_alt[l] = nullptr;
+        }
+        return false;
+    }
+    use_wide(h, true);
+    for (int l = 1; l < h->nl; l++) enqueue_stencil(h, l);
+    err = factor_coarsest_enqueue(h);
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
+    if (err == H3D_OK && e != cudaSuccess) err = fail(h, H3D_ERR_CUDA, cudaGetErrorString(e));
+    if (err == H3D_OK && factor_coarsest_check(h) == H3D_OK) return true;
+    use_wide(h, false);
+    return false;
+}
+
+// A V-cycle whose estimate falls tenfold a cycle and then grows geometrically has lost a
+// coarse mode to the FP16 stencils (a few designs in a thousand; with FP32 stencils the
+// same designs converge in 4 to 9 cycles).  Growing: the estimate rose in two cycles
+// running, to 1.3 times the smallest one since the start.
+struct Trend {
+    double last[2] = {HUGE_VAL, HUGE_VAL}, low = HUGE_VAL;
+    bool growing(double w) {
+        const bool g = w > last[0] && last[0] > last[1] && w > 1.3 * low;
+        last[1] = last[0];
+        last[0] = w;
+        low = std::min(low, w);
+        return g;
+    }
+};
+
 // The solve loop of MG::solveEquation (MG.cpp:113-203) as a resumable state
 // machine: begin() enqueues the first step on the handle's stream; after that
 // stream has drained, advance() reads the step's result and enqueues the next
@@ -474,13 +587,19 @@ namespace {
 // is folded into u64 and the residual recomputed exactly once the estimate has
 // dropped by theta (10x above that floor) or reached the tolerance, and the solve
 // only stops when that exact residual meets the tolerance too.
+//
+// FP16 coarse stencils make the V-cycle diverge on a few high-contrast designs.  Once
+// the estimate grows (Trend, above ten times the FP32 floor), or has exploded twice, the
+// coarse levels are rebuilt with FP32 stencils and the solve goes on from its iterate (or
+// from zero); only if that explodes too does it give up.
 struct SolveRun {
     enum Pending { P_NONE, P_START_REFINE, P_CYCLE, P_TRIGGER_REFINE, P_FINAL_REFINE, P_DONE };
     h3d_handle *h = nullptr;
     int mask = 63, it = 0, nref = 0, status = H3D_OK, explode_left = 2, maxit = 200;
     double tol = 1e-2, theta = 1e-3;
     bool refine = false, exact = false, with_guess = false, fallback_tried = false, done_flag = false;
-    bool u64_zero = false;
+    bool u64_zero = false, widen_next = false;
+    Trend trend;
     double fn[6] = {}, rel[6] = {1, 1, 1, 1, 1, 1}, base[6] = {1, 1, 1, 1, 1, 1};
     // largest selected stale estimate of each cycle since the last refinement
     std::vector<double> since_refine;
@@ -515,12 +634,56 @@ struct SolveRun {
     int launch_cycle() {
         u64_zero = false;
         if (it >= maxit) return finish(H3D_NOT_CONVERGED);
-        CK(cudaGraphLaunch(h->sgraph, h->stream));
+        CK(cudaGraphLaunch(h->sgraph[h->wide], h->stream));
         pending = P_CYCLE;
         return H3D_OK;
     }
     void read_base() {
         for (int c = 0; c < NCASE; c++) base[c] = std::sqrt(h->h_small[c]) / (fn[c] + 1e-10);
+    }
+    int restart_from_zero() {
+        trend = Trend();
+        if (!refine) launch_pin_fold(h->lv[0], h->rho, h->ke, h->pin_state, h->stream);  // restores f
+        if (int e = reset_solution()) return e;
+        CK(cudaMemsetAsync(h->pin_state + NF, 0, sizeof(double) * NF, h->stream));
+        fallback_tried = true;
+        if (refine) {
+            CK(cudaMemsetAsync(h->lv[0].u, 0, sizeof(float) * nf32(), h->stream));
+            return launch_refine(P_START_REFINE);
+        }
+        enqueue_pin_init(h);
+        return launch_cycle();
+    }
+    // FP32 stencils from here on; done is false where they cannot be had
+    int widen(bool &done) {
+        int e = H3D_OK;
+        done = widen_stencils(h, e);
+        if (e) return e;
+        return done ? build_graph(h, G_SOLVE) : H3D_OK;
+    }
+    // Go on alone with a lockstep design that needs FP32 stencils, from its iterate or
+    // (restart) from zero: the state a single solve would be in at this cycle.
+    int adopt(h3d_handle *hh, double tolerance, double theta_, const double fnorm[6], const double r[6], int cycles,
+              int explosions_left, bool restart) {
+        h = hh;
+        tol = tolerance;
+        theta = theta_;
+        it = cycles;
+        explode_left = restart ? 1 : explosions_left;
+        for (int c = 0; c < NCASE; c++) {
+            fn[c] = fnorm[c];
+            rel[c] = r[c];
+        }
+        CK(cudaMemsetAsync(h->d_botflag, 0, sizeof(int), h->stream));
+        h->h_small[61] = 0.0;
+        if (!h->tuned)
+            if (int e = autotune(h)) return e;
+        bool ok = false;
+        if (int e = widen(ok)) return e;
+        if (!ok && restart) return finish(H3D_DIVERGED);
+        if (!ok)  // no memory: the FP16 cycles go on
+            if (int e = build_graph(h, G_SOLVE)) return e;
+        return restart ? restart_from_zero() : launch_cycle();
     }
     // a solve that ends without converging still leaves its iterate in u64; the
     // FP32 solution takes the pending shift and f is restored
@@ -600,6 +763,11 @@ struct SolveRun {
 
     // the step enqueued last has completed on the handle's stream
     int advance() {
+        const int e = step();
+        if (e != H3D_OK) use_wide(h, false);
+        return e;
+    }
+    int step() {
         switch (pending) {
         case P_START_REFINE: {
             read_base();
@@ -634,26 +802,32 @@ struct SolveRun {
             // cycles has met the FP32 floor of its own equation (high-contrast
             // designs): refresh it from the exact residual instead of waiting for theta
             since_refine.push_back(worst);
+            double worst_base = 0;
+            for (int c = 0; c < NCASE; c++)
+                if (selected(c)) worst_base = std::max(worst_base, base[c]);
+            const bool growing = trend.growing(worst) && worst > theta * worst_base && can_widen(h);
             const size_t ns = since_refine.size();
             if (ns >= 4 && !(worst < 0.5 * since_refine[ns - 4])) trigger = true;
-            if (bad) {  // MG.cpp:140-182: restart from zero once, then give up
-                if (--explode_left <= 0) return finish(H3D_DIVERGED);
-                if (!refine) launch_pin_fold(h->lv[0], h->rho, h->ke, h->pin_state, h->stream);  // restores f
-                if (int e = reset_solution()) return e;
-                CK(cudaMemsetAsync(h->pin_state + NF, 0, sizeof(double) * NF, h->stream));
-                fallback_tried = true;
-                if (refine) {
-                    CK(cudaMemsetAsync(h->lv[0].u, 0, sizeof(float) * nf32(), h->stream));
-                    return launch_refine(P_START_REFINE);
+            if (bad) {  // MG.cpp:140-182: restart from zero once (and once with FP32 stencils), then give up
+                if (--explode_left <= 0) {
+                    bool done = false;
+                    if (can_widen(h))
+                        if (int e = widen(done)) return e;
+                    if (!done) return finish(H3D_DIVERGED);
+                    explode_left = 1;
                 }
-                enqueue_pin_init(h);
-                return launch_cycle();
+                return restart_from_zero();
             }
-            if (refine && trigger) {
+            if (refine && (trigger || growing)) {
                 done_flag = done;
+                widen_next = growing;
                 return launch_refine(P_TRIGGER_REFINE);
             }
             if (done) return finish(H3D_OK);
+            if (growing) {
+                bool ok;
+                if (int e = widen(ok)) return e;
+            }
             return launch_cycle();
         }
         case P_TRIGGER_REFINE: {
@@ -663,6 +837,11 @@ struct SolveRun {
                 for (int c = 0; c < NCASE; c++)
                     if (selected(c) && !(base[c] <= tol)) done = false;
             if (done) return finish(H3D_OK);
+            if (widen_next) {
+                widen_next = false;
+                bool ok;
+                if (int e = widen(ok)) return e;
+            }
             return launch_cycle();
         }
         case P_FINAL_REFINE:
@@ -677,6 +856,7 @@ struct SolveRun {
 
     int end(h3d_solve_stats *stats) {
         CK(cudaEventSynchronize(h->ev1));
+        use_wide(h, false);  // the handle's hierarchy is the configured one between solves
         if (stats) {
             stats->vcycles = it;
             stats->refinements = nref;
@@ -690,39 +870,6 @@ struct SolveRun {
         return H3D_OK;
     }
 };
-
-
-// the coarsest level's assembly and Gauss-Jordan inversion with the
-// singular-matrix flag copied to the host; factor_coarsest_check reads it once
-// the stream has drained
-int factor_coarsest_enqueue(h3d_handle *h) {
-    cudaStream_t s = h->stream;
-    if (!h->fgraph) {
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        launch_coarse_assemble(h->lv[h->nl - 1], h->aug, s);
-        cudaMemsetAsync(h->d_flag, 0, sizeof(int), s);
-        launch_gauss_jordan(h->aug, h->ndof, h->d_flag, s);
-        CK(cudaStreamEndCapture(s, &g));
-        cudaError_t e = cudaGraphInstantiate(&h->fgraph, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
-            h->fgraph = nullptr;
-            return fail(h, H3D_ERR_CUDA, std::string("graph: ") + cudaGetErrorString(e));
-        }
-    }
-    CK(cudaGraphLaunch(h->fgraph, s));
-    CK(cudaMemcpyAsync(&h->h_small[63], h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    return H3D_OK;
-}
-
-int factor_coarsest_check(h3d_handle *h) {
-    int flag = 0;
-    std::memcpy(&flag, &h->h_small[63], sizeof(int));
-    if (flag) return fail(h, H3D_ERR_SINGULAR, "coarsest-grid matrix is singular");
-    h->have_stencils = true;
-    return H3D_OK;
-}
 
 // right-hand sides and warm start from the stored solutions, mean removed
 // (homogenization.cu:471-477, grid.cpp:1131-1141)
@@ -910,7 +1057,9 @@ int h3d_destroy(h3d_handle *h) {
     destroy_graph(h);
     for (int l = 0; l < h->nl; l++) {
         cudaFree(h->lv[l].u); cudaFree(h->lv[l].f); cudaFree(h->lv[l].r); cudaFree(h->lv[l].st);
+        cudaFree(h->st_alt[l]);
     }
+    cudaFree(h->aug_alt);
     cudaFree(h->rho); cudaFree(h->chi); cudaFree(h->u64); cudaFree(h->f0);
     cudaFree(h->q); cudaFree(h->d_ked); cudaFree(h->aug);
     cudaFree(h->d_dcw);
@@ -970,12 +1119,10 @@ int h3d_restrict_stencil(h3d_handle *h, int coarse_level) {
     CK(cudaSetDevice(h->device));
     if (coarse_level == 1) {
         if (!h->have_density) return fail(h, H3D_ERR_STATE, "no density");
-        launch_galerkin_l1(h->lv[0], h->lv[1], h->rho, h->q, h->nsub, h->stream);
-        launch_dirichlet_patch(h->lv[0], h->lv[1], h->rho, h->d_ked, h->cfg.pin_mode == H3D_PIN_IDENTITY,
-                               h->stream);
-    } else {
-        launch_galerkin(h->lv[coarse_level - 1], h->lv[coarse_level], h->stream);
     }
+    const unsigned from = coarse_level > 1 ? h->custom >> (coarse_level - 1) & 1u : 0u;
+    h->custom = (h->custom & ~(1u << coarse_level)) | from << coarse_level;
+    enqueue_stencil(h, coarse_level);
     CKL();
     h->have_stencils = false;
     return H3D_OK;
@@ -1609,6 +1756,10 @@ struct LockRun {
     double tol = 1e-2, theta = 1e-3;
     double fn[6] = {}, rel[6] = {1, 1, 1, 1, 1, 1};
     bool live = false;
+    Trend trend;
+    // left the batch to go on alone with FP32 stencils (SolveRun::adopt), from its
+    // iterate or (restart) from zero
+    bool handoff = false, restart = false;
 
     // before the first batch cycle, on the design's stream: balanced right-hand
     // side, reference norms (to the host mirror), deflation state (SolveRun::begin
@@ -1647,13 +1798,23 @@ struct LockRun {
     int advance(const double *norms, cudaStream_t s) {
         it++;
         bool bad = false, done = true;
+        double worst = 0;
         for (int c = 0; c < NCASE; c++) {
             rel[c] = std::sqrt(norms[c]) / (fn[c] + 1e-10);
             if (!(rel[c] <= 10.0)) bad = true;
             if (!(rel[c] <= tol)) done = false;
+            worst = std::max(worst, rel[c]);
         }
+        const bool growing = trend.growing(worst) && worst > theta;
+        const bool fallback = can_widen(h);
         if (bad) {  // MG.cpp:140-182: restart from zero once, then give up
-            if (--explode_left <= 0) return finish(H3D_DIVERGED, s);
+            if (--explode_left <= 0) {
+                if (!fallback) return finish(H3D_DIVERGED, s);
+                handoff = restart = true;
+                live = false;
+                return H3D_OK;
+            }
+            trend = Trend();
             launch_pin_fold(h->lv[0], h->rho, h->ke, h->pin_state, s);  // restores f
             CK(cudaMemsetAsync(h->lv[0].u, 0, sizeof(float) * field_floats(h->lv[0].P.nv), s));
             CK(cudaMemsetAsync(h->pin_state + NF, 0, sizeof(double) * NF, s));
@@ -1661,6 +1822,10 @@ struct LockRun {
             CKL();
         } else if (done) {
             return finish(H3D_OK, s);
+        } else if (growing && fallback) {
+            handoff = true;
+            live = false;
+            return H3D_OK;
         }
         if (it >= maxit) return finish(H3D_NOT_CONVERGED, s);
         return H3D_OK;
@@ -1793,6 +1958,26 @@ int h3d_lockstep_elastic_matrix(h3d_lockstep *b, double tol, double *C, h3d_solv
         }
     }
     LCK(cudaStreamSynchronize(b->stream));
+    for (int i = 0; i < n; i++) {  // the designs that FP16 stencils make diverge, one by one
+        if (!runs[i].handoff) continue;
+        h3d_handle *h = b->hs[i];
+        SolveRun alone;
+        st[i] = [&]() -> int {
+            if (int e = alone.adopt(h, tol, runs[i].theta, runs[i].fn, runs[i].rel, runs[i].it, runs[i].explode_left,
+                                    runs[i].restart))
+                return e;
+            while (!alone.finished()) {
+                CK(cudaStreamSynchronize(h->stream));
+                if (int e = alone.advance()) return e;
+            }
+            CK(cudaStreamSynchronize(h->stream));
+            return H3D_OK;
+        }();
+        use_wide(h, false);
+        runs[i].it = alone.it;
+        runs[i].status = alone.status;
+        for (int c = 0; c < NCASE; c++) runs[i].rel[c] = alone.rel[c];
+    }
     for (int i = 0; i < n; i++) {
         h3d_handle *h = b->hs[i];
         if (st[i] != H3D_OK) continue;
@@ -2055,6 +2240,7 @@ int h3d_set_field(h3d_handle *h, int level, int field, const float *host) {
         launch_stencil_from_lex(L, h->tmp, h->stream);
         CKL();
         CK(cudaStreamSynchronize(h->stream));
+        h->custom |= 1u << level;
         return H3D_OK;
     }
     const size_t n18 = (size_t)NF * L.P.nv, nf = (size_t)field_floats(L.P.nv);

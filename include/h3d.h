@@ -42,7 +42,8 @@ typedef enum {
     H3D_ERR_CUDA = 2,         /* a CUDA call failed; see h3d_last_error */
     H3D_ERR_NOMEM = 3,        /* device allocation failed */
     H3D_NOT_CONVERGED = 4,    /* iteration cap reached above the tolerance */
-    H3D_DIVERGED = 5,         /* relative residual above 10 twice, or NaN */
+    H3D_DIVERGED = 5,         /* relative residual above 10 twice, or NaN (with FP16 stencils
+                                 built from the density: a third time, with FP32 ones) */
     H3D_ERR_STATE = 6,        /* call order violated (e.g. solve before density) */
     H3D_ERR_SINGULAR = 7      /* coarsest-grid matrix could not be inverted */
 } h3d_status;
@@ -81,10 +82,12 @@ typedef enum {
 
 /* storage of the Galerkin coarse-level stencils */
 typedef enum {
-    H3D_STENCIL_FP16 = 0,       /* FP16 entries, images summed in FP16, as the reference does */
-    H3D_STENCIL_FP32 = 1        /* FP32 entries (twice the stencil bytes); keeps the V-cycle
-                                   convergent on high-contrast designs where FP16 rounding of
-                                   the coarse operators stalls or diverges it */
+    H3D_STENCIL_FP16 = 0,       /* FP16 entries, images summed in FP16, as the reference does;
+                                   a solve whose residual estimate grows (a few designs in a
+                                   thousand: FP16 rounding of the coarse operators) goes on
+                                   with FP32 entries to its end, if they fit into memory
+                                   (976 bytes per coarse vertex, kept by the handle) */
+    H3D_STENCIL_FP32 = 1        /* FP32 entries (twice the stencil bytes) from the start */
 } h3d_stencil_precision;
 
 typedef struct {
