@@ -137,9 +137,11 @@ __device__ __forceinline__ void wn_cta_sums(const float *g, float *out) {
 // Weight gradients, dW[co][ci][t] += sum_b sum_v dz[b][co][v] x[b][ci][v + off(t)] and
 // db[co] += sum dz[b][co][v], in two stages: CTA (co group, ci, chunk) sums its chunk of
 // the batch's voxels for WN_GCO output channels (27 x values and WN_GCO dz values for
-// 27 WN_GCO FMAs), k_wn_grad_finish adds the chunks in order.  One CTA per (co, ci)
-// over all voxels left most of the chip idle and loaded a value per FMA: 0.33 ms per
-// layer of the 32^3 network, batch 4; 0.06 ms now.
+// 27 WN_GCO FMAs), k_wn_grad_finish adds the chunks in order and in FP64 (in FP32 the
+// hundreds of chunks of a wide level put the output layer 2e-7 off, 5e-8 now; one chain
+// of 1024 voxels per thread, as before the split, 8e-8).  One CTA per (co, ci) over all
+// voxels left most of the chip idle and loaded a value per FMA: 0.33 ms per layer of the
+// 32^3 network, batch 4; 0.06 ms now.
 constexpr int WN_GCO = 4;
 constexpr int WN_GROW = 28 * WN_GCO;  // partial row: [WN_GCO][27 taps, bias]
 __global__ void __launch_bounds__(WN_BS) k_wn_conv3_wgrad(const float *__restrict__ x, const float *__restrict__ dz,
@@ -180,10 +182,10 @@ __global__ void __launch_bounds__(WN_BS) k_wn_grad_finish(const float *__restric
     const int row = i / WN_GROW, e = i % WN_GROW, t = e % 28;
     const int ci = row % Cin, co = row / Cin * WN_GCO + e / 28;
     if (t == 27 && ci != 0) return;
-    float v = 0.f;
+    double v = 0;
     for (int k = 0; k < nchunk; ++k) v += __ldg(part + ((long long)k * nrow) * WN_GROW + i);
-    if (t < 27) dW[((long long)co * Cin + ci) * 27 + t] += v;
-    else db[co] += v;
+    if (t < 27) dW[((long long)co * Cin + ci) * 27 + t] += (float)v;
+    else db[co] += (float)v;
 }
 
 // 1x1 output layer: y[b][o][v] = bias[o] + sum_c W[o][c] x[b][c][v]
@@ -248,11 +250,11 @@ __global__ void __launch_bounds__(WN_BS) k_wn_out_finish(const float *__restrict
                                                         int nchunk) {
     const int i = blockIdx.x * WN_BS + threadIdx.x, n = Cout * (WN_OIN + 1);
     if (i >= n) return;
-    float v = 0.f;
+    double v = 0;
     for (int k = 0; k < nchunk; ++k) v += __ldg(part + (long long)k * n + i);
     const int o = i / (WN_OIN + 1), c = i % (WN_OIN + 1);
-    if (c < WN_OIN) dW[o * WN_OIN + c] += v;
-    else db[o] += v;
+    if (c < WN_OIN) dW[o * WN_OIN + c] += (float)v;
+    else db[o] += (float)v;
 }
 
 // dz = dy * (y > 0), in place on dy
