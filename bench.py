@@ -160,11 +160,13 @@ def max_over_ranks(dist, value):
     return float(t.item())
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the eight colour
-# launches of one fine sweep: an ncu capture at 128^3 (1.51 GB per sweep: every
-# colour launch reads the whole u field, which exceeds L2) scaled by the vertex
-# count, 3.3x the algorithmic bytes
-SWEEP_TRAFFIC_BYTES = {128: 1_510_000_000, 256: 12_080_000_000}
+# launches of one fine sweep (two of the eight colours each)
+SWEEP_LAUNCHES = 4
+
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the launches of one fine
+# sweep: an ncu capture at 128^3 (0.886 GB per sweep: every launch reads the whole u
+# field, which exceeds L2) scaled by the vertex count, 1.9x the algorithmic bytes
+SWEEP_TRAFFIC_BYTES = {128: 886_000_000, 256: 7_090_000_000}
 
 PRECISION_NAME = {0: "FP32 V-cycles on the correction of an FP64 solution (iterative refinement)",
                   1: "FP32 solution (the reference's scheme)",
@@ -183,9 +185,9 @@ def launches_per_step(nl, vcycles, reso, refine, refinements, coarsest_nv, mixed
     of u64 += u and the FP64 residual (2)"""
     nblk = reso * reso                                          # fine residual norm partials, one per row
     finish = 2 if nblk > 4096 else 1                            # one- or two-stage norm reduction
-    fine = 4 + 1 + finish + 4                                   # GS (two colours per launch), residual, norms, GS
+    fine = 2 * SWEEP_LAUNCHES + 1 + finish                      # GS, residual, norms, GS
     if mixed:
-        fine = 4 + 1 + 1 + 4                                    # GS, tensor-core residual, norms, GS
+        fine = 2 * SWEEP_LAUNCHES + 1 + 1                       # GS, tensor-core residual, norms, GS
     coarse = (nl - 2) * (8 + 1 + 8)                             # GS per colour, residual, GS per colour
     per_cycle = fine + coarse + 2 * (nl - 1) + 1 + 1            # restrict, prolong, coarsest apply, deflation
     per_refine = 1 + 1 + 2 + 3                                  # u64 += u, residual64, norms, deflation restart
@@ -345,7 +347,8 @@ def gpu_arm(args):
                              "frac": round(bpv1 * nv1 / (sweep1_ms * 1e-3) / 1e9 / peaks.get("hbm_gbs"), 4)},
             "gpu_launches": sum(launches_per_step(hd.nlevels, c, args.reso, args.precision != 1, r, coarsest_nv,
                                                   args.precision == 3) for c, r in zip(cycles, refs)),
-            "roofline": {"kernel": "k_fine_gs (8 colour launches = one sweep)", "bound": "hbm",
+            "roofline": {"kernel": "k_fine_gs (%d launches of two colours = one sweep)" % SWEEP_LAUNCHES,
+                         "bound": "hbm", "limited_by": "load latency and instruction issue",
                          "achieved": round(achieved, 1), "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
                          "frac": round(achieved / peaks.get("hbm_gbs"), 4),
                          "traffic": SWEEP_TRAFFIC_BYTES.get(args.reso) if args.precision == 0 else None,
