@@ -229,8 +229,8 @@ __device__ __forceinline__ void prefetch_field(const float *f, unsigned long lon
 }
 
 // ---- vertex pairs --------------------------------------------------------------
-// Rows of a CTA of at most `tmax` threads: whole rows of h0 pairs, `rows` of them, on
-// rows * h0 of its threads (a multiple of 32), chosen to leave the fewest threads idle.
+// A CTA holds whole rows of h0 pairs, `rows` of them, on rows * h0 of its threads (a
+// multiple of 32), chosen to leave the fewest threads idle.
 struct PairShape {
     int rows, threads;
 };
@@ -530,9 +530,9 @@ __global__ void __launch_bounds__(TM, MB) k_fine_gs(FineArgs a, const __grid_con
 // Residual of all rows in one launch (there is no order between colours), the row
 // parity the block index modulo 4 and a run-time value of one code body: the CTAs of
 // neighbouring rows run together and read each other's rows while they are in L2.
-// 256^3: 3.48 ms with one vertex per thread (2.95 ms without the last colour, which the
-// sweep then wrote), 2.47 ms now; three cases per thread or other register budgets
-// measured 2.73 to 3.26.
+// 256^3: 3.48 ms with one vertex per thread (2.95 to 3.06 ms without the last colour,
+// which the sweep then wrote), 2.37 ms now back to back and 2.59 ms with the norms and a
+// cold cache; three cases per thread or other register budgets measured 2.73 to 3.26.
 // norm partials: the six weighted squared norms of every row of vertices, row
 // K0/2 * (rows of a parity) + row, summed in an order that depends on the row length
 // alone (the same in any launch shape and in lockstep batches).
@@ -786,7 +786,8 @@ static void fine_gs_sweep(const FineArgs &a, const KeMat &ke, unsigned nt, cudaS
     k_fine_gs<6, C, TM, MB><<<nb, nt, 0, s>>>(a, ke);
 }
 
-// CTAs of up to 128, 256 or 512 threads (pair_shape), with the same threads per SM
+// CTAs of up to 128, 256 or 512 threads (pair_shape): MB, half of it (rounded down) or
+// one per SM; the register budgets of longer rows differ from the shape's own
 template <int C, int MB>
 static void fine_gs_shape(const FineArgs &a, const KeMat &ke, cudaStream_t s) {
     const unsigned nt = (unsigned)pair_shape(a.h[0]).threads;

@@ -363,7 +363,8 @@ __global__ void __launch_bounds__(256) k_coarse_assemble(Planes C, const uint4 *
 // The factorisation is a serial chain of n pivot steps, bound by their latency: one
 // launch per pivot column over [K | I] took 7.3 us a step (1.41 ms for 192 unknowns,
 // 5.9 ms for 648); here a panel's steps stay inside one CTA.
-// The pivot is the largest |a_ij| to 20 mantissa bits, the first of equals.
+// The pivot is the largest |a_ij| to 20 mantissa bits; of equals the lowest row with one
+// row per thread, the one of the lowest thread with two.
 constexpr int GJ_ROWS_PER_WARP = 4;  // rows of a tile per warp
 
 struct GjArgs {

@@ -15,9 +15,12 @@
 // an element then take about 780 FMAs after 430 additions, where Ke U for six cases
 // alone is 3456.  On the tensor cores (TF32 hi + lo, three products) the dense
 // contraction had to stage operands in shared memory and read the products back from
-// TMEM with 8 warps per SM: 5.25 ms at 256^3, 0.67 ms at 128^3 for C, 0.86 ms at 128^3 for
-// the sensitivities.  chi is FP64 and taken relative to the element's first node before
-// it is rounded to FP32.  Bound by the 144 gathered FP64 values and issue.
+// TMEM with 8 warps per SM.  C at 256^3 / 128^3: 5.23 / 0.67 -> 2.18 / 0.29 ms; a
+// sensitivity call at 256^3 / 128^3 / 64^3: 6.90 / 0.91 / 0.131 -> 2.13 / 0.30 / 0.065 ms.
+// chi is FP64 and taken relative to the element's first node before it is rounded to
+// FP32; C is 2.8e-8 from 64 bits where the split operands were 3.6e-7.  Bound by the 144
+// gathered FP64 values: at 128^3 the L1 data pipe is 51 % busy, issue 43 %, DRAM 19 %,
+// with 8 warps per SM (233 registers) waiting on loads.
 #include <stdint.h>
 
 #include "h3d_internal.cuh"

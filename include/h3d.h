@@ -188,10 +188,12 @@ H3D_API int h3d_reset_solutions(h3d_handle *h);
 
 /* ---- autotuner (no reference counterpart) ----------------------------------
  * Each smoothed level has H3D_NUM_SHAPES launch shapes for its colour sweep and
- * (coarse levels) its residual: load cases per thread (all six, or two as three
- * threads per vertex) times CTAs per SM (the register budget per thread).  Level 0:
- * shape 0 / 1 / 2 / 3 = six cases at 4 CTAs/SM / two at 5 / three at 5 / two at 6;
- * coarse levels: two at 6 / six at 4 / two at 4 / six at 3.  All give the same
+ * (coarse levels) its residual: load cases per thread (a vertex, or on level 0 a pair
+ * of vertices, is then served by one to three threads) times CTAs of 128 threads per SM
+ * (the register budget per thread).  Level 0: shape 0 / 1 / 2 / 3 = three cases at 4
+ * CTAs/SM / six at 2 / two at 5 / three at 3 (rows of more than 256 vertices, or that
+ * fill 128 threads badly, run in CTAs of up to 256 or 512 threads with half as many or
+ * one per SM); coarse levels: two at 6 / six at 4 / two at 4 / six at 3.  All give the same
  * results to the last bit.  The first solve of a handle times them (CUDA events,
  * a few sweeps per shape, iterating on the level's scratch residual field) and
  * keeps the fastest; h3d_autotune re-runs that now, h3d_set_tuning fixes the
@@ -249,8 +251,8 @@ H3D_API int h3d_lockstep_create(h3d_handle *const *hs, int n, h3d_lockstep **out
 H3D_API int h3d_lockstep_create_groups(h3d_handle *const *hs, int n, int groups, h3d_lockstep **out);
 H3D_API int h3d_lockstep_elastic_matrix(h3d_lockstep *b, double tol, double *C, h3d_solve_stats *stats,
                                         int *status);
-/* The sweeps of each group and level run in one of two launch shapes (level 0: six
- * or three load cases per thread; coarse levels: two or six), shape 0 by default;
+/* The sweeps of each group and level run in one of two launch shapes (level 0: three
+ * or two load cases per thread; coarse levels: two or six), shape 0 by default;
  * results do not depend on the shapes.  h3d_lockstep_set_shapes forces every group
  * and level to fine_shape / coarse_shape (0 or 1); h3d_lockstep_autotune times both
  * shapes level by level with the sweeps of all groups running together on scratch

@@ -1,6 +1,6 @@
-"""The element-energy contraction on the tensor cores (k_homog_tc.cu) against the
+"""The element energies (k_homog.cu) against the
 FP64 oracle: sensitivities of arbitrary stored solutions (including a grid whose
-element count is not a multiple of the 128-element tile) and C of solved fields."""
+element count is not a multiple of a CTA's 128) and C of solved fields."""
 import numpy as np
 import pytest
 
