@@ -389,12 +389,20 @@ __device__ __forceinline__ bool pair_task(const FineArgs &a, unsigned rb, int &s
 
 // the reference's component-wise block Gauss-Seidel step (x, then y, then z,
 // each with the relaxed values of the earlier components) written as an
-// update of u by the residual r = f - K u; rk: w over the diagonal of ks
-__device__ __forceinline__ void gs_step(const float ks[9], const float rk[3], float r0, float r1, float r2, float &u0,
-                                        float &u1, float &u2) {
-    const float d0 = r0 * rk[0];
-    const float d1 = (r1 - ks[3] * d0) * rk[1];
-    const float d2 = (r2 - ks[6] * d0 - ks[7] * d1) * rk[2];
+// update of u by the residual r = f - K u; rk: the reciprocals of ks's diagonal.  The
+// quotients are corrected by their remainder (Markstein, IBM J. Res. Dev. 34, 1990, 111),
+// which gives the division's result; the bare product is 3 to 5 % further from 64 bits
+// over a sweep.  Sweep at 256^3 / 128^3 / 64^3: 2.30 / 0.329 / 0.0590 ms with the product,
+// 2.34 / 0.336 / 0.0612 here, 2.44 / 0.352 / 0.0648 with divisions.
+__device__ __forceinline__ float quotient(float a, float b, float rb) {
+    const float q = a * rb;
+    return fmaf(fmaf(-b, q, a), rb, q);
+}
+__device__ __forceinline__ void gs_step(const float ks[9], const float rk[3], float w, float r0, float r1, float r2,
+                                        float &u0, float &u1, float &u2) {
+    const float d0 = quotient(w * r0, ks[0], rk[0]);
+    const float d1 = quotient(w * (r1 - ks[3] * d0), ks[4], rk[1]);
+    const float d2 = quotient(w * (r2 - ks[6] * d0 - ks[7] * d1), ks[8], rk[2]);
     u0 += d0;
     u1 += d1;
     u2 += d2;
@@ -409,7 +417,7 @@ __device__ __forceinline__ void gs_step(const float ks[9], const float rk[3], fl
 // fetched 17 row halves per 128 vertices from L2; this reads u four times and 18 row
 // halves per 256 vertices.  Bound by load latency and issue (54-58 % of issue slots,
 // 15 warps per SM, DRAM 29 % at 128^3).  Sweep at 256^3 / 128^3 / 64^3: 2.82 / 0.42 / 0.082
-// ms with one colour per launch, 2.29 / 0.33 / 0.060 ms now.
+// ms with one colour per launch, 2.34 / 0.34 / 0.061 ms now.
 // bid: the CTA's index in the design's launch; sm: 3 C x TM floats
 template <int K0, int C, int TM>
 __device__ __forceinline__ void fine_gs_block(const FineArgs &a, const KeMat &ke, unsigned bid) {
@@ -473,11 +481,11 @@ __device__ __forceinline__ void fine_gs_block(const FineArgs &a, const KeMat &ke
 #pragma unroll
         for (int e = 0; e < 9; ++e) ks[e] = A[e].x;
 #pragma unroll
-        for (int m = 0; m < 3; ++m) rk[m] = a.w / ks[4 * m];
+        for (int m = 0; m < 3; ++m) rk[m] = 1.f / ks[4 * m];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             float u0 = -nuv[3 * c].x, u1 = -nuv[3 * c + 1].x, u2 = -nuv[3 * c + 2].x;
-            gs_step(ks, rk, fo[3 * c * FVB] - acc[3 * c].x, fo[(3 * c + 1) * FVB] - acc[3 * c + 1].x,
+            gs_step(ks, rk, a.w, fo[3 * c * FVB] - acc[3 * c].x, fo[(3 * c + 1) * FVB] - acc[3 * c + 1].x,
                     fo[(3 * c + 2) * FVB] - acc[3 * c + 2].x, u0, u1, u2);
             sm[3 * c][threadIdx.x] = u0;
             sm[3 * c + 1][threadIdx.x] = u1;
@@ -494,7 +502,7 @@ __device__ __forceinline__ void fine_gs_block(const FineArgs &a, const KeMat &ke
     for (int e = 0; e < 9; ++e) ks[e] = A[e].y;
     g.block(ke, 12, A);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) rk[m] = a.w / ks[4 * m];
+    for (int m = 0; m < 3; ++m) rk[m] = 1.f / ks[4 * m];
     const bool pinned = origin && i == 0;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
@@ -513,7 +521,7 @@ __device__ __forceinline__ void fine_gs_block(const FineArgs &a, const KeMat &ke
             v[r] = fmaf(B[3 * r].y, dr[0], fmaf(B[3 * r + 1].y, dr[1], fmaf(B[3 * r + 2].y, dr[2], v[r])));
         }
         float u0 = -nuv[3 * c].y, u1 = -nuv[3 * c + 1].y, u2 = -nuv[3 * c + 2].y;
-        gs_step(ks, rk, fe[3 * c * FVB] - v[0], fe[(3 * c + 1) * FVB] - v[1], fe[(3 * c + 2) * FVB] - v[2], u0, u1, u2);
+        gs_step(ks, rk, a.w, fe[3 * c * FVB] - v[0], fe[(3 * c + 1) * FVB] - v[1], fe[(3 * c + 2) * FVB] - v[2], u0, u1, u2);
         // the pinned origin stays zero (grid.cu:445-447, 545)
         ue[3 * c * FVB] = pinned ? 0.f : u0;
         ue[(3 * c + 1) * FVB] = pinned ? 0.f : u1;
@@ -775,8 +783,8 @@ static unsigned pair_blocks(const FineArgs &a) { return (unsigned)((a.h[1] * a.h
 int fine_residual_blocks(const Level &L) { return L.P.n[1] * L.P.n[2]; }
 
 // The colour sweep in launch shape v: load cases per thread and CTAs of 128 threads
-// per SM; all give the same result to the last bit (256^3 / 64^3: shape 0 2.29 / 0.060,
-// 1 2.50 / 0.058, 2 2.61 / 0.066, 3 2.57 / 0.065 ms)
+// per SM; all give the same result to the last bit (256^3 / 64^3: shape 0 2.34 / 0.061,
+// 1 2.65 / 0.058, 2 2.63 / 0.067, 3 2.55 / 0.066 ms)
 template <int C, int TM, int MB>
 static void fine_gs_sweep(const FineArgs &a, const KeMat &ke, unsigned nt, cudaStream_t s) {
     const unsigned nb = pair_blocks(a) * (NCASE / C);
