@@ -106,12 +106,11 @@ def test_weighted_norms(torch_cuda):
 
 
 def test_vcycle_fused_residual_paths_match_separate_launches(torch_cuda):
-    """The V-cycle's down leg lets the last colour launch of each level's sweep
-    write that colour's residual and runs the residual launch over the other seven
-    colours (fine and coarse levels).  The same cycle driven through the per-level
-    entry points (a whole sweep, then the residual of all eight colours) must give
-    the same residual on every smoothed level and the same final level-0 field, to
-    FP32 rounding."""
+    """The V-cycle's down leg starts every coarse level from zero: a colour's launch writes
+    its residual so far and the residual launch takes the later colours' share from it.
+    The same cycle driven through the per-level entry points (a cleared level, a whole
+    sweep, then the residual of all eight colours) must give the same residual on every
+    smoothed level and the same final level-0 field, to FP32 rounding."""
     n = 32
     hd, _, t = make_pair(torch_cuda, n=n, seed=5)
     h2 = H.Homogenization(n)
