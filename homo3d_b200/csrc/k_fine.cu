@@ -34,9 +34,14 @@ constexpr int CPT = 2;            // load cases per thread of the FP32 residual
 constexpr int RES_MINB = 4;       // its CTAs of 128 threads per SM
 // Row blocks between a CTA of the pair kernels and the one whose rows it brings into L2.
 // Both kernels wait on loads with few warps (128 registers: 4 CTAs/SM), and more than
-// half of their L1 misses went on to DRAM.  Measured at 256^3: the sweep 2.60 ms without
-// prefetch, 2.36 / 2.32 / 2.29 / 2.29 ms at 150 / 100 / 50 / 20 row blocks, the residual
-// 2.72 ms without, 2.60 / 2.51 / 2.50 / 2.47 at 150 / 50 / 25 / 10.
+// half of their L1 misses went on to DRAM.  Sweep / residual in us without prefetch, and
+// at distances of 5, 20, 60 and 200 for both:
+//   256^3  2666 / 3009    2328 / 2367   2320 / 2369   2330 / 2387   2449 / 2591
+//   192^3  1198 / 1362    1089 / 1097   1089 / 1097   1092 / 1098   1107 / 1116
+//   128^3   366 /  381     334 /  303    333 /  300    337 /  301    352 /  322
+//    96^3   185 /  179     173 /  144    173 /  145    175 /  146    179 /  152
+//    64^3    59 /   43      58 /   43     58 /   43     58 /   43     58 /   43
+// and no difference at 32^3, where the fields stay in L2.
 constexpr unsigned GS_AHEAD = 20, RES_AHEAD = 10;
 constexpr int CPT64 = 2;          // load cases per thread of the FP64-solution residual
 constexpr int MINB64 = 4;         // its CTAs per SM
